@@ -48,8 +48,9 @@ int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, 
                               void *y, int y_cstride, int y_coff, float *yf, const float *resid,
                               const void *mask, int mask_cstride, int mask_coff, void *stream);
 /* 3x3x3 layers whose planes are at least 16 x 8 voxels and whose packed
- * weights and input halo fit in 227 KB of shared memory run on the
- * halo-staged kernel, and the weight gradients of 3x3x3 layers with at most
+ * weights and input halo fit in 227 KB of shared memory run on the z-walk
+ * kernel (at most 80 output channels) or the halo-staged kernel (the same
+ * bits), and the weight gradients of 3x3x3 layers with at most
  * 40 output and 80 input channels on the TMA-staged tap-stacked kernel;
  * enable = 0 sends every layer to the per-tap gather kernels.  Returns the
  * previous setting. */
