@@ -50,13 +50,13 @@ int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, 
 /* 3x3x3 layers whose planes are at least 16 x 8 voxels and whose packed
  * weights and input halo fit in 227 KB of shared memory run on the z-walk
  * kernel (at most 80 output channels) or the halo-staged kernel (the same
- * bits), and the weight gradients of 3x3x3 layers with at most
- * 40 output and 80 input channels on the TMA-staged tap-stacked kernel;
+ * bits), and the weight gradients of 3x3x3 layers with at most 64 output and
+ * 112 input channels on the tap-stacked kernels;
  * enable = 0 sends every layer to the per-tap gather kernels.  Returns the
  * previous setting. */
 int sepx_unet_set_halo(int enable);
 /* Weight-gradient kernel choice (with the halo-staged kernels enabled):
- * 2 (default) the z-walk tap-stacked kernel (cin <= 48, cout <= 40), else
+ * 2 (default) the ring tap-stacked kernel (cin <= 112, cout <= 64), else
  * the per-tile tap-stacked kernel (cin <= 80, cout <= 40), else the gather
  * kernel; 1 the per-tile kernel, else gather; 0 gather.  Returns the
  * previous choice, or -1 for another value. */

@@ -86,6 +86,27 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same, issued by the lanes with lead != 0 (one, from elect_one): the warp's
+// control flow stays uniform, so that descriptors are formed in uniform
+// registers (inside a branch of one lane every operand is moved there first).
+__device__ __forceinline__ void mma_bf16_if(uint32_t lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit_if(uint32_t lead, uint32_t mbar_smem) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(mbar_smem),
+      "r"(lead)
+      : "memory");
+}
 // the mbarrier completes one phase once every MMA issued so far by this thread is done
 __device__ __forceinline__ void mma_commit(uint32_t mbar_smem) {
   asm volatile(

@@ -13,9 +13,9 @@
 //
 // GEMM shapes: forward / data gradient  M = voxels (tiles of 128),
 // N = output channels (16..128), K = taps x input channels (chunks of 64);
-// weight gradient of the narrow layers (sepx_unet_wgrad.inc): M = (x shift,
-// output channel), N = (y shift, input channel), K = the 128 voxels of a
-// tile, nine taps per MMA; of the others (gather kernel below): M = taps x
+// weight gradient (sepx_unet_wgring.inc, cin <= 112 and cout <= 64): M = (x
+// shift, output channel), N = (z shift, input channel), K = the 128 voxels of
+// a tile, nine taps per MMA; of the others (gather kernel below): M = taps x
 // input channels (tiles of 128), N = output channels, K = voxels (chunks of
 // 64, split over CTAs).  Both write per-CTA partial sums that a second kernel
 // adds in a fixed order (the gather kernel adds with FP32 atomics only when
@@ -802,6 +802,8 @@ __global__ void __launch_bounds__(kUThreads) conv_wgrad_kernel(
 
 #include "sepx_unet_wgrad.inc"
 
+#include "sepx_unet_wgring.inc"
+
 // ---------------------------------------------------------------------------
 // Weight packing.  w: FP32 master weights in the weight-gradient layout
 // [ntap][cin_p][cout] (row m = t*cin_p + c).  Forward operand
@@ -1283,7 +1285,7 @@ int np_of(int cout) { return ((cout + 15) / 16) * 16; }
 // shared memory a CTA may have (one CTA per SM for the largest of them).
 constexpr size_t kHaloMaxSmem = 227 * 1024;
 bool g_halo_enabled = true;
-int g_wgrad_form = 2;   // 2: z-walk, else per-tile TMA, else gather; 1: per-tile TMA, else gather; 0: gather
+int g_wgrad_form = 2;   // 2: ring, else per-tile TMA, else gather; 1: per-tile TMA, else gather; 0: gather
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 int g_num_sms = 0;
 size_t g_smem_per_sm = 0, g_smem_reserved = 0;
@@ -1495,86 +1497,90 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
 }
 
-// The z-walk form of the tap-stacked weight gradient (sepx_unet_wgrad.inc)
-// for cin <= 48 and 8 ngo <= 40.  Returns 1 where it does not apply.
-int conv_wgrad_zw(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
-                  const void *dy, int dy_cstride, int dy_coff, int cout, float *dw, float *db, int *err,
-                  cudaStream_t st) {
+// The ring form of the tap-stacked weight gradient (sepx_unet_wgring.inc) for
+// cin <= 112 and cout <= 64.  Returns 1 where it does not apply.
+int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
+                    const void *dy, int dy_cstride, int dy_coff, int cout, float *dw, float *db, int *err,
+                    cudaStream_t st) {
   const int ngi = cin / 8, ngo = (cout + 7) / 8;
-  if (!g_halo_enabled || g_wgrad_form < 2 || 3 * ngo > 16 || ngi > 6) return 1;
+  if (!g_halo_enabled || g_wgrad_form < 2 || ngi > 14 || ngo > 8) return 1;
   if (unet_dev_init()) return -1;
-  ZwArgs a;
+  RgArgs a;
+  a.x = View{(const __nv_bfloat16 *)x, x_cstride, x_coff};
+  a.dy = View{(const __nv_bfloat16 *)dy, dy_cstride, dy_coff};
+  if (reinterpret_cast<uintptr_t>(a.x.p + x_coff) % 16 || reinterpret_cast<uintptr_t>(a.dy.p + dy_coff) % 16)
+    return set_error("unet wgrad: view not 16-byte aligned");
   a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.ngi = ngi; a.ngo = ngo;
-  a.np = ((8 * (3 * ngi + 1)) + 15) / 16 * 16;
-  if (3 * a.np > 512) return 1;
-  a.a_bytes = 3u * ngo * kWgBox;
-  a.pl_bytes = (uint32_t)(a.np / 8) * kWgBox;
-  a.rawb_bytes = 18u * 8u * (uint32_t)cin * 2u;
-  a.rawa_bytes = 16u * 10u * 8u * (uint32_t)ngo * 2u;
-  a.raw_bytes = (a.rawb_bytes + a.rawa_bytes + 127u) / 128u * 128u;
-  const size_t fixed = 2 * (size_t)a.a_bytes + 4 * (size_t)a.pl_bytes + (2 * kZwMaxRaw + 12) * 8 + 16 + 128;
-  if (fixed + 2 * (size_t)a.raw_bytes > kHaloMaxSmem) return 1;
-  uint32_t ncols = 32;
-  while (ncols < (uint32_t)(3 * a.np)) ncols <<= 1;
-  // raw slots: as many as keep the most CTAs per SM (by shared and tensor memory)
-  auto per_sm_of = [&](int nr) {
-    const size_t sm = fixed + (size_t)nr * a.raw_bytes;
+  a.nmbt = (24 * ngo + 127) / 128;
+  // N is a multiple of 16 (of 8 for 64 rows) and at most 256
+  a.stacked = 24 * ngi <= 256 && (ngi % 2 == 0 || (a.nmbt == 1 && rg_mrows(ngo, 0) == 64));
+  a.n = a.stacked ? 24 * ngi : (8 * ngi + 15) / 16 * 16;
+  const int ncn = a.stacked ? a.n : 3 * a.n;
+  // as much of a tile's work per CTA as the tensor memory holds: fewer CTAs
+  // read the same planes
+  a.nsy = a.nmbt * 3 * ncn <= 512 ? 3 : 1;
+  a.nmb = a.nmbt * a.nsy * ncn <= 512 ? a.nmbt : 1;
+  if (a.nmb * a.nsy * ncn > 512) return 1;
+  int ncols = 32;
+  while (ncols < a.nmb * a.nsy * ncn) ncols <<= 1;
+  // pads that spread the groups of neighbouring lanes over the banks
+  auto pad = [](int groups) { return groups <= 2 ? 64 : (groups <= 4 ? 32 : 16); };
+  a.gx = 18 * 8 * 16 + pad(ngi);
+  a.ga = 16 * 8 * 16 + pad(ngo);
+  auto per_sm_of = [&](int na, int nring) {
+    const size_t sm = rg_smem_bytes(ngi, ngo, a.gx, a.ga, na, nring);
     if (sm > kHaloMaxSmem) return 0;
-    const int k = (int)(g_smem_per_sm / (((sm + 127) / 128) * 128 + g_smem_reserved));
-    return std::min(k, 512 / (int)ncols);
+    return std::min((int)(g_smem_per_sm / (((sm + 127) / 128) * 128 + g_smem_reserved)), 512 / ncols);
   };
-  a.nraw = 2;
-  for (int nr = 3; nr <= kZwMaxRaw; nr++)
-    if (per_sm_of(nr) >= per_sm_of(a.nraw)) a.nraw = nr;
-  const size_t smem = fixed + (size_t)a.nraw * a.raw_bytes;
+  // two CTAs per SM where eight planes and three dY operands fit twice, else
+  // one; then the longest ring (four planes at least)
+  int per_sm = per_sm_of(3, 8) >= 2 ? 2 : 1;
+  a.na = per_sm_of(3, 7) >= per_sm ? 3 : 2;
+  a.nring = kRgMaxRing;
+  while (a.nring > 4 && per_sm_of(a.na, a.nring) < per_sm) a.nring--;
+  if (per_sm_of(a.na, a.nring) < per_sm) return 1;
+  a.ty = (H + 15) / 16;
+  a.tx = (W + 2 + 7) / 8;
+  const int njob = (3 / a.nsy) * (a.nmbt / a.nmb);
+  const int slots = std::max(1, g_num_sms * per_sm / njob);
+  // planes per window: the run with the least work on the busiest CTA (a
+  // window loads two planes more than it has tiles; counted half a tile each)
+  const long long cols = (long long)nb * a.ty * a.tx;
+  if (cols * D >= (1LL << 31)) return 1;
+  double best = 1e300;
+  for (int zc = 1; zc <= D; zc++) {
+    const int nzc = (D + zc - 1) / zc;
+    if (zc > 1 && (D + nzc - 1) / nzc != zc) continue;   // windows as even as the count allows
+    const long long per = (cols * nzc + slots - 1) / slots;
+    const double cost = (double)per * (zc + 1.0);
+    if (cost <= best) {
+      best = cost;
+      a.zc = zc;
+      a.nzc = nzc;
+    }
+  }
+  a.nitems = (int)(cols * a.nzc);
+  a.groups = std::min(a.nitems, slots);
+  a.err = err;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_zw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kHaloMaxSmem);
     if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
     attr = true;
   }
-  const int per_sm = per_sm_of(a.nraw);
-  if (per_sm < 1) return 1;
-  const long long slots = (long long)g_num_sms * per_sm;
-  a.ty = (H + 15) / 16;
-  a.tx = (W + 2 + 7) / 8;
-  // planes per window: few windows leave SMs idle, short ones reload more
-  // planes (zc + 2 per zc tiles); take the z run with the least work on the
-  // busiest CTA, counting a plane as a third of a tile
-  const long long cols = (long long)nb * a.ty * a.tx;
-  double best = 1e300;
-  for (int zc = D;; zc = (zc + 1) / 2) {
-    const long long nzc = (D + zc - 1) / zc;
-    const long long items = cols * nzc;
-    const long long per = (items + slots - 1) / slots;
-    const double cost = (double)per * (zc + 2.0 / 3.0);
-    if (cost < best) {
-      best = cost;
-      a.zc = zc;
-      a.nzc = (int)nzc;
-    }
-    if (zc <= 4) break;
-  }
-  a.nitems = cols * a.nzc;
-  if (a.nitems >= (1LL << 31)) return 1;
-  const long long grid = a.nitems < slots ? a.nitems : slots;
-  a.err = err;
-  a.mrows = 3 * 8 * ngo <= 64 ? 64 : 128;
-  CUtensorMap tmx, tmy;
-  if (encode_view(&tmx, x, x_cstride, x_coff, cin, nb, D, H, W, 8, 18, 1, "wgrad x", cin) ||
-      encode_view(&tmy, dy, dy_cstride, dy_coff, 8 * ngo, nb, D, H, W, 10, 16, 1, "wgrad dy", 8 * ngo))
-    return -1;
   const long long n = 27LL * cin * cout;
   float *scr;
-  if (unet_scratch(kScrGrad, (size_t)grid * (size_t)(n + cout), &scr, st)) return -1;
+  if (unet_scratch(kScrGrad, (size_t)a.groups * (size_t)(n + cout), &scr, st)) return -1;
   a.part = scr;
-  a.bpart = scr + (size_t)grid * n;
-  conv_wgrad_zw_kernel<<<(unsigned)grid, kZwThreads, smem, st>>>(tmx, tmy, a);
+  a.bpart = db ? scr + (size_t)a.groups * n : nullptr;
+  conv_wgrad_ring_kernel<<<(unsigned)(a.groups * njob), kRgThreads,
+                           rg_smem_bytes(ngi, ngo, a.gx, a.ga, a.na, a.nring), st>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
-  wg_reduce_kernel<<<(unsigned)((n + cout + 31) / 32), 32 * kRedSlices, 0, st>>>(a.part, (int)grid, n, dw,
-                                                                             a.bpart, cout, db);
+  const long long tot = n + (db ? cout : 0);
+  wg_reduce_kernel<<<(unsigned)((tot + 31) / 32), 32 * kRedSlices, 0, st>>>(a.part, a.groups, n, dw, a.bpart,
+                                                                          db ? cout : 0, db);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet wgrad: %s", cudaGetErrorString(e));
 }
@@ -1861,8 +1867,8 @@ int sepx_unet_conv_wgrad_bias(const void *x, int x_cstride, int x_coff, int nb, 
   if (V >= (1LL << 31) || (long long)H * W * x_cstride >= (1LL << 30))
     return set_error("unet wgrad: volume too large (%lld voxels)", V);
   if (ntap == 27) {
-    int rc = conv_wgrad_zw(x, x_cstride, x_coff, nb, D, H, W, cin, dy, dy_cstride, dy_coff, cout, dw, db,
-                           err, (cudaStream_t)stream);
+    int rc = conv_wgrad_ring(x, x_cstride, x_coff, nb, D, H, W, cin, dy, dy_cstride, dy_coff, cout, dw, db,
+                             err, (cudaStream_t)stream);
     if (rc <= 0) return rc;
     rc = conv_wgrad_tma(x, x_cstride, x_coff, nb, D, H, W, cin, dy, dy_cstride, dy_coff, cout, dw, db, err,
                         (cudaStream_t)stream);
