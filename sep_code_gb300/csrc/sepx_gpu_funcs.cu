@@ -58,6 +58,7 @@ struct Ctx {
   int *d_err = nullptr;
   PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   int zchunk_override = 0;
+  int zc_auto[7] = {0, 0, 0, 0, 0, 0, 0};   // auto_zchunk's choice per mode on this grid (0: not made)
   // modes (bit per PropMode) that run the two-row tile (32 x 32 cells per
   // CTA): none by default -- on GB300 at 560 x 560 x 496 it measured slower
   // than the one-row tile for every mode (2 CTAs per SM instead of 4)
@@ -323,22 +324,60 @@ int build_pointmap(PointMapDev &m, const std::vector<int> &loc, int npts, const 
   return 0;
 }
 
-// Planes per CTA along z.  Longer chunks amortise the 8-plane warm-up of the
-// z-queues; shorter ones balance the waves.  Measured on GB300 at 560x560x496:
-// source_prop and the Born forward are best near 80 planes, the RTM adjoint
-// near 32.  Small grids shorten the chunk until there are two waves of
-// 3 CTAs per SM.
+// Planes per CTA along z of a single-grid step: the even split of the depth
+// with the least modelled time.  A wave of r CTAs per SM takes
+// (z (1 + beta (r - 1)) + w) plane times: w planes of start (queues, first
+// copies), beta what another resident CTA costs each.  Measured on grids from
+// 80 x 80 x 128 to 560 x 560 x 496 (3 to 121 planes per CTA, six modes), the
+// choice is within 0.3 to 3 % of the best of each sweep on average; the rule
+// before it (80 planes, 32 for the adjoints, halved while under two waves)
+// ran small grids up to 2.1 times as long (80 x 80 x 128: source propagation
+// 9.6 us a step -> 5.7, adjoint 20.7 -> 9.8; 112 x 112 x 160: 11.3 -> 8.0,
+// 24.0 -> 13.6) and left a last chunk of a few planes on others (448 x 352 x
+// 400: Born forward 407 -> 380).  The limits: chunks beyond 81 planes lose
+// to the caches' reuse of halo rows (560 x 560 x 496: 898 us at 81, 916 at
+// 97), the RTM adjoint's beyond 24 (834 us at 20 to 24, 852 at 32, 889 at 49).
 int auto_zchunk(int mode) {
+  if (G.zchunk_override > 0) return G.zchunk_override;
+  if (G.zc_auto[mode] > 0) return G.zc_auto[mode];
+  const PropGeom &g = G.geom;
+  const long long tiles = (long long)((g.xe - g.xb + kTX - 1) / kTX) * ((g.ye - g.yb + kTY - 1) / kTY);
+  const int depth = std::max(1, g.ze - g.zb);
+  const bool slow_start = mode == kSrcProp || mode == kLinSrc || mode == kLinFwd;
+  const double beta = slow_start ? 0.1 : 0.35, w = slow_start ? 5.0 : 2.5;
+  const int cap = (mode == kRtmAdj || mode == kRtmAdj1) ? 24 : 81;
+  const int per_sm = (mode == kSrcProp || mode == kBornFwd) ? 4 : 3;   // resident CTAs (registers)
+  const long long slots = (long long)per_sm * G.num_sms;
+  double best = 1e300;
+  int zc = 1;
+  for (int n = (depth + cap - 1) / cap; n <= depth; n++) {
+    const int z = (depth + n - 1) / n;
+    const long long ctas = tiles * ((depth + z - 1) / z);
+    const long long full = ctas / slots, rest = (ctas % slots + G.num_sms - 1) / G.num_sms;
+    double t = (double)full * (z * (1.0 + beta * (per_sm - 1)) + w);
+    if (rest) t += z * (1.0 + beta * (double)(rest - 1)) + w;
+    if (t < best) {
+      best = t;
+      zc = z;
+    }
+  }
+  return G.zc_auto[mode] = zc;
+}
+
+// The same for the shots of a batch, which fill the GPU together: 80 planes (32
+// for the adjoints), halved while one shot alone stays under two waves of 3
+// CTAs per SM.
+int batch_zchunk(int mode) {
   if (G.zchunk_override > 0) return G.zchunk_override;
   const PropGeom &g = G.geom;
   const long long tiles = (long long)((g.xe - g.xb + kTX - 1) / kTX) * ((g.ye - g.yb + kTY - 1) / kTY);
   const int depth = std::max(1, g.ze - g.zb);
-  int zc = (mode == kRtmAdj || mode == kRtmAdj1 || mode == kLinAdj) ? 32 : 80;
+  int zc = (mode == kRtmAdj || mode == kRtmAdj1) ? 32 : 80;
   while (zc > 16 && tiles * ((depth + zc - 1) / zc) < 2LL * 3 * G.num_sms) zc /= 2;
   return std::max(1, std::min(zc, depth));
 }
 
-// The same for the two-row tile (32 x 32 cells, 2 CTAs per SM): the chunk
+// The chunk of the two-row tile (32 x 32 cells, 2 CTAs per SM): the chunk
 // count of the target length, planes spread evenly over the chunks.
 int auto_zchunk2(int mode) {
   if (G.zchunk_override > 0) return G.zchunk_override;
@@ -763,6 +802,7 @@ int sepx_create_gpu_space(float d1, float d2, float d3, float bc_a, float bc_b, 
   g.xg = 16 * ((n1 - 8) / 16);
   g.yg = 16 * ((n2 - 8) / 16);
   g.zchunk = 0;
+  for (int &z : G.zc_auto) z = 0;
   if (!same) {
     RET(alloc_volume(G.vel));
     RET(alloc_volume(G.img));
