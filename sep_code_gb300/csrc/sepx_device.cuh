@@ -140,6 +140,19 @@ __device__ __forceinline__ void stcs4(float *p, float4 v) { __stcs(reinterpret_c
 
 __device__ __forceinline__ float4 ldg4(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
 
+// Programmatic dependent launch (launches made with the attribute; without it
+// both return at once): griddep_launch lets the next grid of the stream start
+// as this one's CTAs leave room; griddep_wait blocks until every earlier grid
+// has completed and its writes are visible.  Memory that an earlier grid may
+// still write is read with ldw4 (no read-only path) and only after the wait.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ float4 ldw4(const float *p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ float comp(const float4 &v, int c) {
   return c == 0 ? v.x : (c == 1 ? v.y : (c == 2 ? v.z : v.w));
 }

@@ -397,23 +397,26 @@ __device__ __forceinline__ void run_tile(const PropParams &P, const PropParams &
     // M::TQ: this warp's lanes of the z-queues in tensor memory (allocated by
     // the kernel once, for every tile it runs)
     const uint32_t tq = tq_base + ((uint32_t)(warp * 32) << 16);
-    // warm-up: planes za-4 .. za+3 of the current field(s) along z
+    // warm-up: planes za-4 .. za+3 of the current field(s) along z, the eight
+    // loads of a field in flight together
     if (active || M::TQ) {
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const long long off = rowoff + g.plane * (za - 4 + j);
+      for (int f = 0; f < NF; f++) {
+        float4 w[8];
 #pragma unroll
-        for (int f = 0; f < NF; f++) {
-          float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (active) {
-            p = ldg4(P.cur[f] + off);
-            if (f == 0 && M::F0_VEL_INSIDE) p = mul4(p, ldg4(P.vel + off));
-          }
-          if (M::TQ) {
-            tc::tmem_st4x2_sync(tq + f * 64 + 4 * j, tq + f * 64 + 4 * (j + 8), p);
-          } else {
-            q[f][j] = p;
-          }
+        for (int j = 0; j < 8; j++) {
+          w[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (active) w[j] = ldw4(P.cur[f] + rowoff + g.plane * (za - 4 + j));
+        }
+        if (f == 0 && M::F0_VEL_INSIDE && active) {
+#pragma unroll
+          for (int j = 0; j < 8; j++) w[j] = mul4(w[j], ldg4(P.vel + rowoff + g.plane * (za - 4 + j)));
+        }
+        if constexpr (M::TQ) {
+          tc::tmem_st32x2_sync(tq + f * 64, tq + f * 64 + 32, w);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; j++) q[f][j] = w[j];
         }
       }
     }
@@ -652,12 +655,16 @@ __device__ __forceinline__ void run_tile(const PropParams &P, const PropParams &
 #pragma unroll
             for (int c = 0; c < 4; c++) {
               for (int id = __ldg(mp + c); id >= 0; id = __ldg(P.rec.next + id)) {
+                // the eight samples are distinct: all loads before the
+                // stores (one round trip instead of eight on the planes with
+                // receivers, which small grids wait for)
                 float *tr = P.trc + (long long)P.trc_id * P.nrec + id;
+                float smp[8];
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                  float *a = tr + (long long)k * P.nrec;
-                  *a = __fmaf_rn(xv[c], __ldg(P.sinc_row + k), *a);
-                }
+                for (int k = 0; k < 8; k++) smp[k] = tr[(long long)k * P.nrec];
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                  tr[(long long)k * P.nrec] = __fmaf_rn(xv[c], __ldg(P.sinc_row + k), smp[k]);
               }
             }
           }

@@ -232,6 +232,15 @@ __device__ __forceinline__ void tmem_st4x2_sync(uint32_t a0, uint32_t a1, float4
       "r"(__float_as_uint(v.w))
       : "memory");
 }
+// eight planes at once: q[0..7] to the 32 columns at a0 and to the 32 at a1
+__device__ __forceinline__ void tmem_st32x2_sync(uint32_t a0, uint32_t a1, const float4 (&q)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33};\n\t"
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%1], {%2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33};\n\t"
+      "tcgen05.wait::st.sync.aligned;" ::"r"(a0),
+      "r"(a1), "r"(__float_as_uint(q[0].x)), "r"(__float_as_uint(q[0].y)), "r"(__float_as_uint(q[0].z)), "r"(__float_as_uint(q[0].w)), "r"(__float_as_uint(q[1].x)), "r"(__float_as_uint(q[1].y)), "r"(__float_as_uint(q[1].z)), "r"(__float_as_uint(q[1].w)), "r"(__float_as_uint(q[2].x)), "r"(__float_as_uint(q[2].y)), "r"(__float_as_uint(q[2].z)), "r"(__float_as_uint(q[2].w)), "r"(__float_as_uint(q[3].x)), "r"(__float_as_uint(q[3].y)), "r"(__float_as_uint(q[3].z)), "r"(__float_as_uint(q[3].w)), "r"(__float_as_uint(q[4].x)), "r"(__float_as_uint(q[4].y)), "r"(__float_as_uint(q[4].z)), "r"(__float_as_uint(q[4].w)), "r"(__float_as_uint(q[5].x)), "r"(__float_as_uint(q[5].y)), "r"(__float_as_uint(q[5].z)), "r"(__float_as_uint(q[5].w)), "r"(__float_as_uint(q[6].x)), "r"(__float_as_uint(q[6].y)), "r"(__float_as_uint(q[6].z)), "r"(__float_as_uint(q[6].w)), "r"(__float_as_uint(q[7].x)), "r"(__float_as_uint(q[7].y)), "r"(__float_as_uint(q[7].z)), "r"(__float_as_uint(q[7].w))
+      : "memory");
+}
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, float4 v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr),
                "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)),
