@@ -80,6 +80,13 @@
 #ifndef SEPX_FWD_STAGES
 #define SEPX_FWD_STAGES 2
 #endif
+// packed operations of the modes with the velocity inside the Laplacian (Pk)
+#ifndef SEPX_PK_FWD
+#define SEPX_PK_FWD 0
+#endif
+#ifndef SEPX_PK_LIN
+#define SEPX_PK_LIN 3
+#endif
 #ifndef SEPX_ADJ_STAGES
 #define SEPX_ADJ_STAGES 3
 #endif
@@ -132,6 +139,8 @@ struct Mode {
   static constexpr bool TQ = (SEPX_TMEMQ && MODE == kBornFwd) || (SEPX_TMEMQ_ADJ && MODE == kRtmAdj) ||
                               (SEPX_TMEMQ_LIN && MODE == kLinFwd) || (SEPX_TMEMQ_SP && MODE == kSrcProp);
   static constexpr uint32_t TQ_COLS = NF == 2 ? 128u : 64u;
+  // packed operations (Pk)
+  static constexpr int PK = (MODE == kBornFwd) ? SEPX_PK_FWD : (MODE == kLinFwd ? SEPX_PK_LIN : 7);
   // resident blocks per SM the register budget is sized for
   static constexpr int MINB = (MODE == kSrcProp)  ? SEPX_SP_MINB
                               : (MODE == kBornFwd) ? SEPX_FWD_MINB
@@ -207,66 +216,126 @@ __device__ __forceinline__ float damp_k(float v, float t) {
   return v;
 }
 
-// z-pair sums of a queue (plane z-4+j in qz[j]): zs[k-1] = qz[4+k] + qz[4-k]
-__device__ __forceinline__ void zpairs(const float4 (&qz)[9], float4 (&zs)[4]) {
-#pragma unroll
-  for (int k = 1; k <= 4; k++)
-    zs[k - 1] = make_float4(__fadd_rn(qz[4 + k].x, qz[4 - k].x), __fadd_rn(qz[4 + k].y, qz[4 - k].y),
-                            __fadd_rn(qz[4 + k].z, qz[4 - k].z), __fadd_rn(qz[4 + k].w, qz[4 - k].w));
+// ---- packed arithmetic: columns (0, 1) and (2, 3) of a thread's four cells as
+// two float2 (one instruction adds, multiplies or fuses two FP32 values, each
+// rounded like its scalar form: the same bits).  PK says which operations are
+// packed: 1 additions, 2 fused multiply-adds, 4 products.  The modes that do
+// not multiply by the velocity inside the Laplacian pack all three (step
+// issue-bound before: 128^3 source propagation and adjoint 9.71 -> 9.06 ms for
+// 150 steps, 256^3 linearised adjoint 14.1 -> 13.4 for 60).  The velocity-
+// inside form must not: a packed product whose only use is a packed sum is
+// contracted into one rounding, .rn or not (seen as 1-ulp differences from the
+// oracle); the linearised forward keeps scalar products (64^3 patch 14.8 ->
+// 13.9 ms), and the Born forward, whose 96 registers the pairs overrun, stays
+// scalar (512 x 512 x 400, 60 steps: 53.3 ms, packed sums 54.8) ----
+template <int PK>
+struct Pk {
+  static __device__ __forceinline__ float2 add(float2 a, float2 b) {
+    float2 r;
+    if constexpr ((PK & 1) != 0)
+      asm("{\n\t.reg .b64 a, b, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+          "add.rn.f32x2 r, a, b;\n\tmov.b64 {%0, %1}, r;\n\t}"
+          : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    else
+      r = make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+    return r;
+  }
+  static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) {
+    float2 r;
+    if constexpr ((PK & 2) != 0)
+      asm("{\n\t.reg .b64 a, b, c, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+          "fma.rn.f32x2 r, a, b, c;\n\tmov.b64 {%0, %1}, r;\n\t}"
+          : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    else
+      r = make_float2(__fmaf_rn(a.x, b.x, c.x), __fmaf_rn(a.y, b.y, c.y));
+    return r;
+  }
+  static __device__ __forceinline__ float2 mul(float2 a, float2 b) {
+    float2 r;
+    if constexpr ((PK & 4) != 0)
+      asm("{\n\t.reg .b64 a, b, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+          "mul.rn.f32x2 r, a, b;\n\tmov.b64 {%0, %1}, r;\n\t}"
+          : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    else
+      r = make_float2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+    return r;
+  }
+};
+__device__ __forceinline__ float2 half2of(const float4 &v, int h) {
+  return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+}
+__device__ __forceinline__ float2 dup2(float c) { return make_float2(c, c); }
+__device__ __forceinline__ float4 mul4(const float4 &a, const float4 &b) {
+  return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
 }
 
-// z-pair k of column c: from the 9-plane queue, summed where it is used, or
-// from the pair sums
-__device__ __forceinline__ float zterm(const float4 (&qz)[9], int k, int c) {
-  return __fadd_rn(comp(qz[4 + k], c), comp(qz[4 - k], c));
+// z-pair sums of a queue (plane z-4+j in qz[j]): zs[k-1] = qz[4+k] + qz[4-k]
+template <int PK = 0>
+__device__ __forceinline__ void zpairs(const float4 (&qz)[9], float4 (&zs)[4]) {
+#pragma unroll
+  for (int k = 1; k <= 4; k++) {
+    const float2 l = Pk<PK>::add(half2of(qz[4 + k], 0), half2of(qz[4 - k], 0)),
+                 h = Pk<PK>::add(half2of(qz[4 + k], 1), half2of(qz[4 - k], 1));
+    zs[k - 1] = make_float4(l.x, l.y, h.x, h.y);
+  }
 }
-__device__ __forceinline__ float zterm(const float4 (&zs)[4], int k, int c) {
-  return comp(zs[k - 1], c);
+
+// z-pair k, half h: from the 9-plane queue, summed where it is used, or from
+// the pair sums
+template <int PK>
+__device__ __forceinline__ float2 zterm(const float4 (&qz)[9], int k, int h) {
+  return Pk<PK>::add(half2of(qz[4 + k], h), half2of(qz[4 - k], h));
+}
+template <int PK>
+__device__ __forceinline__ float2 zterm(const float4 (&zs)[4], int k, int h) { return half2of(zs[k - 1], h); }
+
+// x-pair k of half h of a row window w (columns x-4 .. x+7): the two columns'
+// w[+k] + w[-k].  For odd k the operands straddle register pairs: two scalar
+// adds cost less than the moves that would pair them up.
+template <int PK>
+__device__ __forceinline__ float2 xpair(const float (&w)[12], int k, int h) {
+  const int i = 4 + 2 * h;
+  if (k & 1) return make_float2(__fadd_rn(w[i + k], w[i - k]), __fadd_rn(w[i + 1 + k], w[i + 1 - k]));
+  return Pk<PK>::add(make_float2(w[i + k], w[i + 1 + k]), make_float2(w[i - k], w[i + 1 - k]));
 }
 
 // Laplacian part of wave_kernel (vel outside): s = c0 p + sum_k pairs.
 // xw: x-4 .. x+7 of the row, ym/yp: rows y-k / y+k, zq: the z-queue (plane
 // z-4+j in zq[j]) or its pair sums.
-template <int NZ>
+template <int PK, int NZ>
 __device__ __forceinline__ void lap_plain(const float *coef, const float (&xw)[12],
                                           const float4 (&ym)[4], const float4 (&yp)[4],
-                                          const float4 (&zq)[NZ], float (&s)[4]) {
+                                          const float4 (&zq)[NZ], float2 (&s)[2]) {
 #pragma unroll
-  for (int c = 0; c < 4; c++) {
-    float p = xw[4 + c];
-    float acc = __fmul_rn(coef[0], p);
+  for (int h = 0; h < 2; h++) {
+    float2 acc = Pk<PK>::mul(dup2(coef[0]), make_float2(xw[4 + 2 * h], xw[5 + 2 * h]));
 #pragma unroll
     for (int k = 1; k <= 4; k++) {
-      acc = __fmaf_rn(coef[3 * k - 2], __fadd_rn(xw[4 + c + k], xw[4 + c - k]), acc);
-      acc = __fmaf_rn(coef[3 * k - 1], __fadd_rn(comp(yp[k - 1], c), comp(ym[k - 1], c)), acc);
-      acc = __fmaf_rn(coef[3 * k], zterm(zq, k, c), acc);
+      acc = Pk<PK>::fma(dup2(coef[3 * k - 2]), xpair<PK>(xw, k, h), acc);
+      acc = Pk<PK>::fma(dup2(coef[3 * k - 1]), Pk<PK>::add(half2of(yp[k - 1], h), half2of(ym[k - 1], h)), acc);
+      acc = Pk<PK>::fma(dup2(coef[3 * k]), zterm<PK>(zq, k, h), acc);
     }
-    s[c] = acc;
+    s[h] = acc;
   }
 }
 
 // Laplacian of (v p), wave_kernel_adj (vel inside): centre (c0 p) v, pairs of
-// rounded products; zq: z-queue of the products p v, or its pair sums.
-template <int NZ>
-__device__ __forceinline__ void lap_velin(const float *coef, const float (&xw)[12],
-                                          const float (&vw)[12], const float4 (&ym)[4],
-                                          const float4 (&yp)[4], const float4 (&vym)[4],
-                                          const float4 (&vyp)[4], const float4 (&zq)[NZ],
-                                          float (&s)[4]) {
+// rounded products (xw, ym, yp already hold them); zq: z-queue of the
+// products p v, or its pair sums.
+template <int PK, int NZ>
+__device__ __forceinline__ void lap_velin(const float *coef, const float4 &p, const float4 &v,
+                                          const float (&xw)[12], const float4 (&ym)[4],
+                                          const float4 (&yp)[4], const float4 (&zq)[NZ], float2 (&s)[2]) {
 #pragma unroll
-  for (int c = 0; c < 4; c++) {
-    float acc = __fmul_rn(__fmul_rn(coef[0], xw[4 + c]), vw[4 + c]);
+  for (int h = 0; h < 2; h++) {
+    float2 acc = Pk<PK>::mul(Pk<PK>::mul(dup2(coef[0]), half2of(p, h)), half2of(v, h));
 #pragma unroll
     for (int k = 1; k <= 4; k++) {
-      float px = __fadd_rn(__fmul_rn(xw[4 + c + k], vw[4 + c + k]),
-                           __fmul_rn(xw[4 + c - k], vw[4 + c - k]));
-      acc = __fmaf_rn(coef[3 * k - 2], px, acc);
-      float py = __fadd_rn(__fmul_rn(comp(yp[k - 1], c), comp(vyp[k - 1], c)),
-                           __fmul_rn(comp(ym[k - 1], c), comp(vym[k - 1], c)));
-      acc = __fmaf_rn(coef[3 * k - 1], py, acc);
-      acc = __fmaf_rn(coef[3 * k], zterm(zq, k, c), acc);
+      acc = Pk<PK>::fma(dup2(coef[3 * k - 2]), xpair<PK>(xw, k, h), acc);
+      acc = Pk<PK>::fma(dup2(coef[3 * k - 1]), Pk<PK>::add(half2of(yp[k - 1], h), half2of(ym[k - 1], h)), acc);
+      acc = Pk<PK>::fma(dup2(coef[3 * k]), zterm<PK>(zq, k, h), acc);
     }
-    s[c] = acc;
+    s[h] = acc;
   }
 }
 
@@ -281,11 +350,6 @@ __device__ __forceinline__ void load_window(const float *h, float (&w)[12], floa
     ym[k - 1] = lds4(h + 4 - k * kHX);
     yp[k - 1] = lds4(h + 4 + k * kHX);
   }
-}
-
-__device__ __forceinline__ float4 mul4(float4 a, float4 b) {
-  return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z),
-                     __fmul_rn(a.w, b.w));
 }
 
 // Shared-memory carve of one CTA: [STAGES stages][full bars][empty bars]
@@ -445,7 +509,7 @@ __device__ __forceinline__ void run_tile(const PropParams &P, const PropParams &
             if (f == 0 && M::F0_VEL_INSIDE) p = mul4(p, lds4(sf + M::FEEDV + coff));
           }
           qf[8] = p;
-          zpairs(qf, zs[f]);
+          zpairs<M::PK>(qf, zs[f]);
           tc::tmem_st4x2_sync(tq + f * 64 + 4 * (i & 7), tq + f * 64 + 4 * ((i & 7) + 8), p);
         }
       } else {
@@ -485,27 +549,45 @@ __device__ __forceinline__ void run_tile(const PropParams &P, const PropParams &
           float xw[12];
           float4 ym[4], yp[4];
           load_window(st + M::HALO + f * kHaloFloats + hoff, xw, ym, yp);
-          float sl[4];
+          const float4 pc = make_float4(xw[4], xw[5], xw[6], xw[7]);
+          float2 sl[2];
           if (f == 0 && M::F0_VEL_INSIDE) {
-            if constexpr (M::TQ)
-              lap_velin(P.coef, xw, vw, ym, yp, vym, vyp, zs[f], sl);
-            else
-              lap_velin(P.coef, xw, vw, ym, yp, vym, vyp, q[f], sl);
 #pragma unroll
-            for (int c = 0; c < 4; c++)
-              res[f][c] = M::INC0 ? sl[c] : __fadd_rn(__fadd_rn(sl[c], xw[4 + c]), xw[4 + c]);
+            for (int i = 0; i < 12; i += 2) {
+              const float2 m = Pk<M::PK>::mul(make_float2(xw[i], xw[i + 1]), make_float2(vw[i], vw[i + 1]));
+              xw[i] = m.x;
+              xw[i + 1] = m.y;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              ym[k] = mul4(ym[k], vym[k]);
+              yp[k] = mul4(yp[k], vyp[k]);
+            }
+            if constexpr (M::TQ)
+              lap_velin<M::PK>(P.coef, pc, velc, xw, ym, yp, zs[f], sl);
+            else
+              lap_velin<M::PK>(P.coef, pc, velc, xw, ym, yp, q[f], sl);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const float2 r = M::INC0 ? sl[h] : Pk<M::PK>::add(Pk<M::PK>::add(sl[h], half2of(pc, h)), half2of(pc, h));
+              res[f][2 * h] = r.x;
+              res[f][2 * h + 1] = r.y;
+            }
           } else {
             if constexpr (M::TQ)
-              lap_plain(P.coef, xw, ym, yp, zs[f], sl);
+              lap_plain<M::PK>(P.coef, xw, ym, yp, zs[f], sl);
             else
-              lap_plain(P.coef, xw, ym, yp, q[f], sl);
+              lap_plain<M::PK>(P.coef, xw, ym, yp, q[f], sl);
 #pragma unroll
-            for (int c = 0; c < 4; c++)
-              res[f][c] = (f == 0 && M::INC0)
-                              ? sl[c]
-                              : __fadd_rn(__fmaf_rn(vwc[c], sl[c], xw[4 + c]), xw[4 + c]);
+            for (int h = 0; h < 2; h++) {
+              const float2 r = (f == 0 && M::INC0)
+                                   ? sl[h]
+                                   : Pk<M::PK>::add(Pk<M::PK>::fma(half2of(velc, h), sl[h], half2of(pc, h)), half2of(pc, h));
+              res[f][2 * h] = r.x;
+              res[f][2 * h + 1] = r.y;
+            }
           }
-          if (f == 0 && M::INC0) cur0 = make_float4(xw[4], xw[5], xw[6], xw[7]);
+          if (f == 0 && M::INC0) cur0 = pc;
           prevv[f] = lds4(st + M::PREV + f * kCenterFloats + coff);
         }
         if (load_img) imgv = lds4(st + M::IMG + coff);
