@@ -540,6 +540,8 @@ int loop_rtm_adjoint(int jt, int npts, int nt) {
   RET(zero_volume(*D1));
   RET(zero_volume(G.img));
   PropParams P = base_params();
+  P.src.map = G.srcmap.map;
+  P.src.next = G.srcmap.next;
   P.rec.plane_slot = G.recmap.plane_slot;
   P.rec.map = G.recmap.map;
   P.rec.next = G.recmap.next;
@@ -547,6 +549,14 @@ int loop_rtm_adjoint(int jt, int npts, int nt) {
   P.nrec = G.rec_nx * G.rec_ny;
   Rows2Maps H;
   H.vel_h = G.vel.tm_h2;
+  // A launch per step for the source values costs about 5 us with its gap; the
+  // fused form costs the step kernel 2 % (a register for the next plane's
+  // slot): 128^3 model 10.24 -> 9.79 ms for 150 steps, 512 x 512 x 400 49.42
+  // -> 50.10 for 40.  The line is where both are about 4 us.
+  const PropGeom &gg = G.geom;
+  const long long cells = (long long)(gg.xe - gg.xb) * (gg.ye - gg.yb) * std::max(0, gg.ze - gg.zb);
+  const bool fused = npts > 0 && cells <= 32000000LL &&
+                     !(((G.rows2_mask >> kRtmAdj) & 1) && prop_step2_supported(kRtmAdj));
   for (int it = nt - 1; it >= 0; it--) {
     const int id = it / jt, ii = it - id * jt;
     P.trc_id = id;
@@ -560,8 +570,14 @@ int loop_rtm_adjoint(int jt, int npts, int nt) {
       set_field(P, 1, *S1, *S0);
       H.cur_h[0] = D1->tm_h2;
       H.cur_h[1] = S1->tm_h2;
+      // the source values of sample it + 1 go into the source field this step
+      // advances from (Born/gpu_funcs_3d.cu:655-675): added by the next step
+      // as it reads that field back, or by a launch of their own
+      const bool pending = fused && it < nt - 2;
+      P.src.plane_slot = pending ? G.srcmap.plane_slot : nullptr;
+      P.inj_s = pending ? G.d_inj + (size_t)(it + 1) * npts : nullptr;
       CKL(launch_step(kRtmAdj, P, &H));
-      if (npts > 0)
+      if (npts > 0 && !fused)
         CKL(launch_point_add(S1->origin, G.srcmap.off, G.d_inj + (size_t)it * npts, npts, G.stream));
       std::swap(S0, S1);
     }
