@@ -12,6 +12,70 @@
 
 namespace sepx {
 
+// What bounds these kernels is the FP64 pipe (2 operations per clock and SM),
+// which also runs the conversions between float and double: with them a dot
+// product of 65.5 M elements took 364 us and y = a x1 + b x2 626 us, 1.4 and
+// 1.3 TB/s.  Conversions are therefore done on the integer units (the same
+// values; a group with anything but normal numbers and zeros takes the
+// conversion instructions), and rows are read and written 16 bytes at a time:
+// one FP64 operation per element is left in the dot product (127 us), two in
+// the scaled sums (265 us).
+
+// subnormal, infinite or NaN
+__device__ __forceinline__ bool f2d_odd(float x) {
+  const uint32_t m = __float_as_uint(x) & 0x7fffffffu;
+  return m - 0x00800000u >= 0x7f000000u && m != 0u;
+}
+// a normal number or a zero as a double
+__device__ __forceinline__ double f2d_int(float x) {
+  const uint32_t u = __float_as_uint(x), m = u & 0x7fffffffu;
+  const uint32_t hi = m ? (m >> 3) + 0x38000000u : 0u;   // exponent bias 127 -> 1023
+  return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)(u << 29));
+}
+// N floats as doubles: the conversion instructions only where one of them needs
+// them, in one real branch (a predicated conversion occupies the pipe all the
+// same; volatile: nothing is hoisted)
+template <int N>
+__device__ __forceinline__ void f2d(const float (&x)[N], double (&d)[N]) {
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < N; i++) odd |= f2d_odd(x[i]);
+  if (__any_sync(__activemask(), odd)) {
+#pragma unroll
+    for (int i = 0; i < N; i++) asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d[i]) : "f"(x[i]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i++) d[i] = f2d_int(x[i]);
+  }
+}
+
+// results outside the normal range of float (or at its upper end, where
+// rounding may leave it), zeros apart
+__device__ __forceinline__ bool d2f_odd(double d) {
+  const uint32_t m = (uint32_t)__double2hiint(d) & 0x7fffffffu;
+  return m - 0x38100000u >= 0x0fd00000u && (m | (uint32_t)__double2loint(d)) != 0u;
+}
+// the others, rounded to the nearest float, ties to even: 29 bits go, half of
+// the last kept bit is added (less one where that bit is even)
+__device__ __forceinline__ float d2f_int(double d) {
+  const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d), m = hi & 0x7fffffffu;
+  const uint64_t r = (((uint64_t)(m - 0x38000000u) << 32) | lo) + 0x0fffffffu + ((lo >> 29) & 1u);
+  return __uint_as_float(((m | lo) ? (uint32_t)(r >> 29) : 0u) | (hi & 0x80000000u));
+}
+template <int N>
+__device__ __forceinline__ void d2f(const double (&d)[N], float (&x)[N]) {
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < N; i++) odd |= d2f_odd(d[i]);
+  if (__any_sync(__activemask(), odd)) {
+#pragma unroll
+    for (int i = 0; i < N; i++) asm volatile("cvt.rn.f32.f64 %0, %1;" : "=f"(x[i]) : "d"(d[i]));
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i++) x[i] = d2f_int(d[i]);
+  }
+}
+
 constexpr int kDotBlocks = 4 * 152;   // 4 CTAs per SM on a 152-SM GB300
 constexpr int kDotThreads = 256;
 
@@ -32,63 +96,168 @@ __device__ __forceinline__ double block_sum(double v) {
 }
 
 // partials[b] = sum over the grid-stride elements of block b of a[i]*b[i]
-// (b == nullptr: sum of a[i])
+// (b == nullptr: sum of a[i]); the block that finishes last adds the partials
+// in block order (a fixed order: repeatable bits) and writes *out, which may
+// be mapped host memory.  done: a counter that is 0 before and after.
+// VEC: both pointers 16-byte aligned, four elements per load.
+template <bool VEC>
 __global__ void __launch_bounds__(kDotThreads)
-    dot_partial_kernel(const float *__restrict__ a, const float *__restrict__ b, long long n,
-                       double *__restrict__ partials) {
-  double acc = 0.0;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-    acc += (double)a[i] * (b ? (double)b[i] : 1.0);
-  acc = block_sum(acc);
-  if (threadIdx.x == 0) partials[blockIdx.x] = acc;
+    dot_kernel(const float *__restrict__ a, const float *__restrict__ b, long long n, double *partials,
+               unsigned int *done, double *out) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  long long i0 = t;
+  if (VEC) {
+    const float4 *a4 = reinterpret_cast<const float4 *>(a), *b4 = reinterpret_cast<const float4 *>(b);
+    const long long n4 = n >> 2;
+    for (long long i = t; i < n4; i += stride) {
+      const float4 x = __ldg(a4 + i);
+      if (b) {
+        const float4 y = __ldg(b4 + i);
+        const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+        double d[8];
+        f2d(v, d);
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[e] += d[e] * d[4 + e];
+      } else {
+        const float v[4] = {x.x, x.y, x.z, x.w};
+        double d[4];
+        f2d(v, d);
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[e] += d[e];
+      }
+    }
+    i0 = (n4 << 2) + t;
+  }
+  for (long long i = i0; i < n; i += stride) acc[0] += (double)a[i] * (b ? (double)b[i] : 1.0);
+  double v = block_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = v;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;   // uniform for the block
+  __threadfence();
+  v = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v += __ldcg(partials + i);
+  __syncthreads();     // block_sum's shared array again
+  v = block_sum(v);
+  if (threadIdx.x == 0) {
+    *out = v;
+    *done = 0u;
+  }
 }
 
-__global__ void __launch_bounds__(kDotThreads)
-    sum_partials_kernel(const double *__restrict__ partials, int np, double *__restrict__ out) {
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) acc += partials[i];
-  acc = block_sum(acc);
-  if (threadIdx.x == 0) *out = acc;
-}
-
-__global__ void fill_kernel(float *x, long long n, float v) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride) x[i] = v;
-}
-
+// ---- elementwise operations on N elements at a time, y = op(y, x1, x2): 8 or 4
+// where every pointer is 16-byte aligned, else (and past the last four) 1 ----
+struct OpFill {
+  float v;
+  template <int N>
+  __device__ void operator()(float (&y)[N], const float (&)[N], const float (&)[N]) const {
+#pragma unroll
+    for (int i = 0; i < N; i++) y[i] = v;
+  }
+};
+// y = y*a (hypercube_float::scale)
+struct OpScale {
+  double a;
+  template <int N>
+  __device__ void operator()(float (&y)[N], const float (&)[N], const float (&)[N]) const {
+    double d[N];
+    f2d(y, d);
+#pragma unroll
+    for (int i = 0; i < N; i++) d[i] *= a;
+    d2f(d, y);
+  }
+};
 // y = y*a + x*b  (hypercube_float::scale_add(a, x, b): vals = vals*a + b*x,
 // Born/hypercube_float.cpp:437-443; evaluated in double as the reference does)
-__global__ void scale_add_kernel(float *y, const float *x, long long n, double a, double b) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-    y[i] = (float)((double)y[i] * a + b * (double)x[i]);
-}
-
+struct OpScaleAdd {
+  double a, b;
+  template <int N>
+  __device__ void operator()(float (&y)[N], const float (&x)[N], const float (&)[N]) const {
+    double d[N], e[N];
+    f2d(y, d);
+    f2d(x, e);
+#pragma unroll
+    for (int i = 0; i < N; i++) d[i] = d[i] * a + b * e[i];
+    d2f(d, y);
+  }
+};
 // y = x1*a + x2*b  (the four-argument scale_add, :368-378)
-__global__ void scale_add2_kernel(float *y, const float *x1, const float *x2, long long n, double a,
-                                  double b) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-    y[i] = (float)((double)x1[i] * a + (double)x2[i] * b);
-}
+struct OpScaleAdd2 {
+  double a, b;
+  template <int N>
+  __device__ void operator()(float (&y)[N], const float (&x1)[N], const float (&x2)[N]) const {
+    double d[N], e[N];
+    f2d(x1, d);
+    f2d(x2, e);
+#pragma unroll
+    for (int i = 0; i < N; i++) d[i] = d[i] * a + e[i] * b;
+    d2f(d, y);
+  }
+};
+struct OpAdd {
+  template <int N>
+  __device__ void operator()(float (&y)[N], const float (&x)[N], const float (&)[N]) const {
+#pragma unroll
+    for (int i = 0; i < N; i++) y[i] = y[i] + x[i];
+  }
+};
+struct OpMult {
+  template <int N>
+  __device__ void operator()(float (&y)[N], const float (&x)[N], const float (&)[N]) const {
+#pragma unroll
+    for (int i = 0; i < N; i++) y[i] = y[i] * x[i];
+  }
+};
 
-__global__ void scale_kernel(float *y, long long n, double a) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-    y[i] = (float)((double)y[i] * a);
-}
-
-__global__ void add_kernel(float *y, const float *x, long long n) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-    y[i] = y[i] + x[i];
-}
-
-__global__ void mult_kernel(float *y, const float *x, long long n) {
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += stride)
-    y[i] = y[i] * x[i];
+template <bool Y, bool X1, bool X2, class OP>
+__global__ void __launch_bounds__(256) map_kernel(float *y, const float *x1, const float *x2, long long n, int vec,
+                                                  OP op) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  long long i0 = t;
+  if (vec) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const long long n4 = n >> 2;
+    // eight elements a step where there are as many: shorter slow paths of the
+    // conversions are predicated instead of branched around
+    long long i = t;
+    for (; i + stride < n4; i += 2 * stride) {
+      float v[8], p[8], q[8];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const long long k = i + h * stride;
+        const float4 a = Y ? reinterpret_cast<const float4 *>(y)[k] : z;
+        const float4 b = X1 ? reinterpret_cast<const float4 *>(x1)[k] : z;
+        const float4 c = X2 ? reinterpret_cast<const float4 *>(x2)[k] : z;
+        v[4 * h] = a.x; v[4 * h + 1] = a.y; v[4 * h + 2] = a.z; v[4 * h + 3] = a.w;
+        p[4 * h] = b.x; p[4 * h + 1] = b.y; p[4 * h + 2] = b.z; p[4 * h + 3] = b.w;
+        q[4 * h] = c.x; q[4 * h + 1] = c.y; q[4 * h + 2] = c.z; q[4 * h + 3] = c.w;
+      }
+      op(v, p, q);
+      reinterpret_cast<float4 *>(y)[i] = make_float4(v[0], v[1], v[2], v[3]);
+      reinterpret_cast<float4 *>(y)[i + stride] = make_float4(v[4], v[5], v[6], v[7]);
+    }
+    if (i < n4) {
+      const float4 a = Y ? reinterpret_cast<const float4 *>(y)[i] : z;
+      const float4 b = X1 ? reinterpret_cast<const float4 *>(x1)[i] : z;
+      const float4 c = X2 ? reinterpret_cast<const float4 *>(x2)[i] : z;
+      float v[4] = {a.x, a.y, a.z, a.w};
+      const float p[4] = {b.x, b.y, b.z, b.w}, q[4] = {c.x, c.y, c.z, c.w};
+      op(v, p, q);
+      reinterpret_cast<float4 *>(y)[i] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    i0 = (n4 << 2) + t;
+  }
+  for (long long i = i0; i < n; i += stride) {
+    float v[1] = {Y ? y[i] : 0.f};
+    const float p[1] = {X1 ? x1[i] : 0.f}, q[1] = {X2 ? x2[i] : 0.f};
+    op(v, p, q);
+    y[i] = v[0];
+  }
 }
 
 // uniform(-0.5, 0.5) from a counter hash (splitmix64) of (seed, index)
@@ -103,44 +272,55 @@ __global__ void random_kernel(float *y, long long n, unsigned long long seed) {
   }
 }
 
+static bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 static int grid_for(long long n) {
   long long g = (n + 255) / 256;
   return (int)(g < 2048 ? (g < 1 ? 1 : g) : 2048);
 }
 
-cudaError_t vec_dot(const float *a, const float *b, long long n, double *partials, double *d_out,
-                    cudaStream_t st) {
-  dot_partial_kernel<<<kDotBlocks, kDotThreads, 0, st>>>(a, b, n, partials);
-  sum_partials_kernel<<<1, kDotThreads, 0, st>>>(partials, kDotBlocks, d_out);
+template <bool Y, bool X1, bool X2, class OP>
+static cudaError_t map(float *y, const float *x1, const float *x2, long long n, OP op, cudaStream_t st) {
+  const int vec = al16(y) && (!X1 || al16(x1)) && (!X2 || al16(x2));
+  map_kernel<Y, X1, X2><<<grid_for(vec ? (n + 7) / 8 : n), 256, 0, st>>>(y, x1, x2, n, vec, op);
   return cudaGetLastError();
 }
 
-int vec_dot_scratch_doubles() { return kDotBlocks; }
+// scratch: vec_dot_scratch_doubles() doubles (partials, then the counter,
+// which must be zero before the first call)
+cudaError_t vec_dot(const float *a, const float *b, long long n, double *scratch, double *out, cudaStream_t st) {
+  unsigned int *done = reinterpret_cast<unsigned int *>(scratch + kDotBlocks);
+  // at least eight elements per thread: few blocks for short vectors, whose
+  // partials the last block waits for
+  const long long want = (n + 8 * kDotThreads - 1) / (8 * kDotThreads);
+  const int blocks = (int)(want < 1 ? 1 : (want > kDotBlocks ? kDotBlocks : want));
+  if (al16(a) && al16(b))
+    dot_kernel<true><<<blocks, kDotThreads, 0, st>>>(a, b, n, scratch, done, out);
+  else
+    dot_kernel<false><<<blocks, kDotThreads, 0, st>>>(a, b, n, scratch, done, out);
+  return cudaGetLastError();
+}
+
+int vec_dot_scratch_doubles() { return kDotBlocks + 1; }
 
 cudaError_t vec_fill(float *x, long long n, float v, cudaStream_t st) {
-  fill_kernel<<<grid_for(n), 256, 0, st>>>(x, n, v);
-  return cudaGetLastError();
+  return map<false, false, false>(x, nullptr, nullptr, n, OpFill{v}, st);
 }
 cudaError_t vec_scale(float *y, long long n, double a, cudaStream_t st) {
-  scale_kernel<<<grid_for(n), 256, 0, st>>>(y, n, a);
-  return cudaGetLastError();
+  return map<true, false, false>(y, nullptr, nullptr, n, OpScale{a}, st);
 }
 cudaError_t vec_scale_add(float *y, const float *x, long long n, double a, double b, cudaStream_t st) {
-  scale_add_kernel<<<grid_for(n), 256, 0, st>>>(y, x, n, a, b);
-  return cudaGetLastError();
+  return map<true, true, false>(y, x, nullptr, n, OpScaleAdd{a, b}, st);
 }
 cudaError_t vec_scale_add2(float *y, const float *x1, const float *x2, long long n, double a, double b,
                            cudaStream_t st) {
-  scale_add2_kernel<<<grid_for(n), 256, 0, st>>>(y, x1, x2, n, a, b);
-  return cudaGetLastError();
+  return map<false, true, true>(y, x1, x2, n, OpScaleAdd2{a, b}, st);
 }
 cudaError_t vec_add(float *y, const float *x, long long n, cudaStream_t st) {
-  add_kernel<<<grid_for(n), 256, 0, st>>>(y, x, n);
-  return cudaGetLastError();
+  return map<true, true, false>(y, x, nullptr, n, OpAdd{}, st);
 }
 cudaError_t vec_mult(float *y, const float *x, long long n, cudaStream_t st) {
-  mult_kernel<<<grid_for(n), 256, 0, st>>>(y, x, n);
-  return cudaGetLastError();
+  return map<true, true, false>(y, x, nullptr, n, OpMult{}, st);
 }
 cudaError_t vec_random(float *y, long long n, unsigned long long seed, cudaStream_t st) {
   random_kernel<<<grid_for(n), 256, 0, st>>>(y, n, seed);

@@ -5,8 +5,9 @@
 namespace sepx {
 
 // FP64 dot product of two float vectors (b == nullptr: sum of a), written to
-// the device double *d_out; `partials` is scratch of vec_dot_scratch_doubles().
-cudaError_t vec_dot(const float *a, const float *b, long long n, double *partials, double *d_out,
+// *out (device or mapped host memory); `scratch`: vec_dot_scratch_doubles()
+// doubles, zero before the first call and used by one stream at a time.
+cudaError_t vec_dot(const float *a, const float *b, long long n, double *scratch, double *out,
                     cudaStream_t st);
 int vec_dot_scratch_doubles();
 cudaError_t vec_fill(float *x, long long n, float v, cudaStream_t st);

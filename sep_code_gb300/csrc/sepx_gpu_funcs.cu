@@ -99,8 +99,8 @@ struct Ctx {
   size_t inj_cap = 0;
   float *d_stage = nullptr;
   size_t stage_cap = 0;
-  double *d_dot = nullptr;    // dot-product partials + result
-  size_t dot_cap = 0;
+  double *d_dot = nullptr;    // dot-product partials and counter
+  double *h_dot = nullptr;    // its result (mapped host memory)
   // compressed source snapshots of the linearised pair
   unsigned char *d_snap = nullptr;
   size_t snap_cap = 0;
@@ -1095,11 +1095,15 @@ int sepx_dot_f32(const float *a, const float *b, long long n, double *result) {
   RET(need_buf(result, "sepx_dot_f32 result"));
   RET(need_span(a, n, "sepx_dot_f32 a"));   // b == NULL: the sum of a
   RET(need_device());
-  const int np = vec_dot_scratch_doubles();
-  RET(ensure(&G.d_dot, &G.dot_cap, (size_t)np + 1));
-  CKL(vec_dot(a, b, n, G.d_dot, G.d_dot + np, G.stream));
-  CK(cudaMemcpyAsync(result, G.d_dot + np, sizeof(double), cudaMemcpyDeviceToHost, G.stream));
+  // the result goes straight to mapped host memory: no copy behind the kernel
+  if (!G.d_dot) {
+    CK(cudaMalloc((void **)&G.d_dot, vec_dot_scratch_doubles() * sizeof(double)));
+    CK(cudaMemsetAsync(G.d_dot, 0, vec_dot_scratch_doubles() * sizeof(double), G.stream));
+  }
+  if (!G.h_dot) CK(cudaHostAlloc((void **)&G.h_dot, sizeof(double), cudaHostAllocMapped));
+  CKL(vec_dot(a, b, n, G.d_dot, G.h_dot, G.stream));
   CK(cudaStreamSynchronize(G.stream));
+  *result = *G.h_dot;
   return 0;
 }
 
