@@ -31,6 +31,16 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   return d;
 }
 
+// K-major operand in the 32-byte swizzle: rows of 32 B (16 BF16), consecutive;
+// the 16-byte halves of a row are exchanged where address bit 7 is set.  The
+// exchange follows the address, so saddr may be any row of a 256-byte aligned
+// area and groups of 8 rows may lie sbo bytes (a multiple of 32) apart
+// (checked on the GPU for row pitches of 8, 10 and 16 voxels and starts up to
+// 22 rows in).
+__device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t saddr, uint32_t sbo) {
+  return smem_desc(saddr, 16, sbo) | ((uint64_t)6 << 61);
+}
+
 // ---- instruction descriptor, kind::f16 with BF16 inputs and FP32 accumulator ----
 // bits 4-5 D format (1 = F32); 7-9 A format (1 = BF16); 10-12 B format
 // (1 = BF16); 15 A major (0 K, 1 MN); 16 B major; 17-22 N >> 3; 24-28 M >> 4.
@@ -132,29 +142,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// two of them behind one wait
-__device__ __forceinline__ void tmem_ld16x2(uint32_t t0, uint32_t t1, float (&v0)[16], float (&v1)[16]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-      "%12, %13, %14, %15}, [%32];\n\t"
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, "
-      "%26, %27, %28, %29, %30, %31}, [%33];\n\t"
-      "tcgen05.wait::ld.sync.aligned;"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(t0), "r"(t1)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; i++) {
-    v0[i] = __uint_as_float(r[i]);
-    v1[i] = __uint_as_float(r[16 + i]);
-  }
-}
-
 // Eight 32-lane x 4-column loads (columns col + 4j .. col + 4j + 3, j = 0..7,
 // each naturally aligned) into q[0..7]; thread t reads lane (32 * (warp % 4)
 // + t).  Loads and the wait in one block: the registers are valid after it.
@@ -239,6 +226,18 @@ __device__ __forceinline__ void tmem_st32x2_sync(uint32_t a0, uint32_t a1, const
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%1], {%2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33};\n\t"
       "tcgen05.wait::st.sync.aligned;" ::"r"(a0),
       "r"(a1), "r"(__float_as_uint(q[0].x)), "r"(__float_as_uint(q[0].y)), "r"(__float_as_uint(q[0].z)), "r"(__float_as_uint(q[0].w)), "r"(__float_as_uint(q[1].x)), "r"(__float_as_uint(q[1].y)), "r"(__float_as_uint(q[1].z)), "r"(__float_as_uint(q[1].w)), "r"(__float_as_uint(q[2].x)), "r"(__float_as_uint(q[2].y)), "r"(__float_as_uint(q[2].z)), "r"(__float_as_uint(q[2].w)), "r"(__float_as_uint(q[3].x)), "r"(__float_as_uint(q[3].y)), "r"(__float_as_uint(q[3].z)), "r"(__float_as_uint(q[3].w)), "r"(__float_as_uint(q[4].x)), "r"(__float_as_uint(q[4].y)), "r"(__float_as_uint(q[4].z)), "r"(__float_as_uint(q[4].w)), "r"(__float_as_uint(q[5].x)), "r"(__float_as_uint(q[5].y)), "r"(__float_as_uint(q[5].z)), "r"(__float_as_uint(q[5].w)), "r"(__float_as_uint(q[6].x)), "r"(__float_as_uint(q[6].y)), "r"(__float_as_uint(q[6].z)), "r"(__float_as_uint(q[6].w)), "r"(__float_as_uint(q[7].x)), "r"(__float_as_uint(q[7].y)), "r"(__float_as_uint(q[7].z)), "r"(__float_as_uint(q[7].w))
+      : "memory");
+}
+// zeros to 16 columns (complete after tmem_wait_st) / 32 columns of the warp's lanes
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(0) : "memory");
+}
+__device__ __forceinline__ void tmem_zero32(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};\n\t"
+      "tcgen05.wait::st.sync.aligned;" ::"r"(taddr),
+      "r"(0)
       : "memory");
 }
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, float4 v) {
