@@ -304,6 +304,7 @@ __global__ void conv_finish_kernel(const float *__restrict__ kpart, int splits, 
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) acc[i] = 0.f;
+#pragma unroll 8
     for (int k = 0; k < splits; k++) {
       const float4 *src = reinterpret_cast<const float4 *>(kpart + ((size_t)k * V + v) * np + n0);
       const float4 a = src[0], b = src[1];
@@ -803,6 +804,8 @@ __global__ void __launch_bounds__(kUThreads) conv_wgrad_kernel(
 #include "sepx_unet_wgrad.inc"
 
 #include "sepx_unet_wgring.inc"
+
+#include "sepx_unet_kstream.inc"
 
 // ---------------------------------------------------------------------------
 // Weight packing.  w: FP32 master weights in the weight-gradient layout
@@ -1498,6 +1501,87 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
 }
 
+// The convolution with streamed weights (sepx_unet_kstream.inc): 3x3x3 layers
+// whose weights do not fit in shared memory or whose planes are smaller than a
+// tile, where channels come in pairs of groups (a K16 step stays in one tap),
+// the planes a K range reads fit in shared memory, and staging them moves at
+// most half of what the gather kernel copies for the range and the tile's real
+// voxels.  Measured (gather -> this, kernel, us): 112 -> 48 on 32^3 voxels 91
+// -> 29, 48 -> 112 on 4 x 16^3 32 -> 19, both beyond the line; short of it (K
+// ranges of 3 chunks) 64 -> 64 on 16^3 10.5 -> 11.2, on 4 x 8^3 8.1 -> 8.8.
+// Returns 1 where it does not apply.
+int conv_kstream(View x, int nb, int D, int H, int W, int cin, const void *wpacked, const float *bias, int cout,
+                 int np, int relu, void *y, int y_cstride, int y_coff, float *yf, const float *resid, View mask,
+                 int *err, int splits, int kper, float *kpart, cudaStream_t st) {
+  if (cin % 16 || cin / 8 > kKsMaxGroups) return 1;
+  KsArgs a;
+  a.ty = (H + kTileY - 1) / kTileY;
+  a.tx = (W + kTileX - 1) / kTileX;
+  const long long cols = (long long)nb * a.ty * a.tx;
+  if (cols * D * splits >= (1LL << 31)) return 1;
+  // planes of one output plane that any range reads
+  int span = 1;
+  const int per9 = 9 * (cin / 16);
+  for (int s = 0; s < splits; s++) {
+    const int k0 = s * kper * (kKC / 16), k1 = std::min(k0 + kper * (kKC / 16), 3 * per9);
+    span = std::max(span, (k1 - 1) / per9 - k0 / per9 + 1);
+  }
+  const double staged = (double)cols * D * span * (kHaloX * kHaloY) * cin, gathered = (double)nb * D * H * W * kper * kKC;
+  if (2 * staged > gathered) return 1;
+  if (unet_dev_init()) return -1;
+  auto fit = [&](int nring, int nw) {
+    const size_t sm = ks_smem_bytes(cin, np, nring, nw);
+    if (sm > kHaloMaxSmem) return 0;
+    return std::min((int)(g_smem_per_sm / ((sm + 127) / 128 * 128 + g_smem_reserved)), 2);
+  };
+  // two CTAs per SM where the planes and two weight slots leave room for them
+  const int want = std::max(fit(span, 2), 1);
+  a.nw = kKsMaxW;
+  while (a.nw > 2 && fit(span, a.nw) < want) a.nw--;
+  const int per_sm = fit(span, a.nw);
+  if (!per_sm) return 1;
+  a.nring = span;
+  while (a.nring < kKsMaxRing && fit(a.nring + 1, a.nw) >= per_sm) a.nring++;
+  // output planes of an item: all ranges of a split layer are items already;
+  // else the count with the fewest planes on the busiest CTA (an item's first
+  // planes cost about half an output plane's MMAs)
+  const long long slots = (long long)g_num_sms * per_sm;
+  a.zc = 1;
+  if (splits == 1) {
+    double best = 1e300;
+    for (int zc = 1; zc <= D; zc++) {
+      const long long items = cols * ((D + zc - 1) / zc);
+      const double c = (double)((items + slots - 1) / slots) * (zc + 0.5);
+      if (c < best) {
+        best = c;
+        a.zc = zc;
+      }
+    }
+  }
+  a.nzc = (D + a.zc - 1) / a.zc;
+  a.zc = (D + a.nzc - 1) / a.nzc;   // the same runs, evenly filled
+  a.nitems = (int)(cols * a.nzc * splits);
+  a.x = x; a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.np = np; a.relu = relu;
+  a.wp = (const __nv_bfloat16 *)wpacked; a.bias = bias;
+  a.y = (__nv_bfloat16 *)y; a.y_cstride = y_cstride; a.y_coff = y_coff;
+  a.yf = yf; a.resid = resid; a.mask = mask; a.err = err;
+  a.splits = splits; a.kper = kper; a.kpart = kpart;
+  static bool attr = false;
+  if (!attr) {
+    cudaError_t e = cudaFuncSetAttribute(conv_kstream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kHaloMaxSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(conv_kstream_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return set_error("unet conv: %s", cudaGetErrorString(e));
+    attr = true;
+  }
+  conv_kstream_kernel<<<(unsigned)std::min<long long>(a.nitems, slots), kKsThreads,
+                        ks_smem_bytes(cin, np, a.nring, a.nw), st>>>(a);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
+}
+
 // The ring form of the tap-stacked weight gradient (sepx_unet_wgring.inc) for
 // cin <= 112 and cout <= 64.  Returns 1 where it does not apply.
 int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
@@ -1826,20 +1910,23 @@ int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, 
     kper = (kch + splits - 1) / splits;
     splits = (kch + kper - 1) / kper;
   }
-  if (splits > 1) {
-    float *kpart;
-    if (unet_scratch(kScrConv, (size_t)splits * V * np, &kpart, (cudaStream_t)stream)) return -1;
+  float *kpart = nullptr;
+  if (splits > 1 && unet_scratch(kScrConv, (size_t)splits * V * np, &kpart, (cudaStream_t)stream)) return -1;
+  int rc = 1;
+  if (ntap == 27 && g_halo_enabled)
+    rc = conv_kstream(xv, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y, y_cstride, y_coff, yf, resid, mv, err,
+                      splits, kper, kpart, (cudaStream_t)stream);
+  if (rc < 0) return rc;
+  if (rc) {
     conv_fwd_kernel<<<dim3((unsigned)mt, (unsigned)splits), kUThreads, smem, (cudaStream_t)stream>>>(
         xv, nb, D, H, W, cin, ntap, (const __nv_bfloat16 *)wpacked, kch, bias, cout, np, relu,
         (__nv_bfloat16 *)y, y_cstride, y_coff, yf, resid, err, kper, kpart, mv);
+  }
+  if (splits > 1) {
     const long long work = V * ((cout + 7) / 8);
     conv_finish_kernel<<<(unsigned)std::min<long long>((work + 255) / 256, 8 * 152), 256, 0,
                          (cudaStream_t)stream>>>(kpart, splits, V, np, bias, cout, relu,
                                                  (__nv_bfloat16 *)y, y_cstride, y_coff, yf, resid, mv);
-  } else {
-    conv_fwd_kernel<<<(unsigned)mt, kUThreads, smem, (cudaStream_t)stream>>>(
-        xv, nb, D, H, W, cin, ntap, (const __nv_bfloat16 *)wpacked, kch, bias, cout, np, relu,
-        (__nv_bfloat16 *)y, y_cstride, y_coff, yf, resid, err, kch, nullptr, mv);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
