@@ -41,6 +41,17 @@ __device__ __forceinline__ uint64_t smem_desc_sw32(uint32_t saddr, uint32_t sbo)
   return smem_desc(saddr, 16, sbo) | ((uint64_t)6 << 61);
 }
 
+// MN-major operand in the swizzle as wide as its rows (one K index each): rows
+// of `channels` = 16, 32 or 64 BF16 (32-, 64- or 128-byte swizzle: the 16-byte
+// units of a row are permuted by address bits 7, 7-8 or 7-9).  atom: bytes
+// between runs of `channels` M/N indices, kgroup: between groups of 8 rows.  As
+// the permutation follows the address, saddr may be any row of a 1024-byte
+// aligned area and atoms may overlap (checked on the GPU for atoms one row
+// apart, groups 8 and 10 rows apart and starts at any row).
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t saddr, uint32_t atom, uint32_t kgroup, int channels) {
+  return smem_desc(saddr, atom, kgroup) | ((uint64_t)(channels == 16 ? 6 : (channels == 32 ? 4 : 2)) << 61);
+}
+
 // ---- instruction descriptor, kind::f16 with BF16 inputs and FP32 accumulator ----
 // bits 4-5 D format (1 = F32); 7-9 A format (1 = BF16); 10-12 B format
 // (1 = BF16); 15 A major (0 K, 1 MN); 16 B major; 17-22 N >> 3; 24-28 M >> 4.

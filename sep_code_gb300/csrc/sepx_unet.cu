@@ -1623,11 +1623,12 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   a.dy = View{(const __nv_bfloat16 *)dy, dy_cstride, dy_coff};
   if (reinterpret_cast<uintptr_t>(a.x.p + x_coff) % 16 || reinterpret_cast<uintptr_t>(a.dy.p + dy_coff) % 16)
     return set_error("unet wgrad: view not 16-byte aligned");
-  a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.ngi = ngi; a.ngo = ngo;
-  a.nmbt = (24 * ngo + 127) / 128;
-  // N is a multiple of 16 (of 8 for 64 rows) and at most 256
-  a.stacked = 24 * ngi <= 256 && (ngi % 2 == 0 || (a.nmbt == 1 && rg_mrows(ngo, 0) == 64));
-  a.n = a.stacked ? 24 * ngi : (8 * ngi + 15) / 16 * 16;
+  a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.ngo = ngo;
+  a.ncb = (ngi + 1) / 2;
+  a.pw = cout <= 16 ? 16 : (cout <= 32 ? 32 : 64);
+  a.nmbt = a.pw == 64 ? 2 : 1;
+  a.stacked = 48 * a.ncb <= 256;
+  a.n = a.stacked ? 48 * a.ncb : 16 * a.ncb;
   const int ncn = a.stacked ? a.n : 3 * a.n;
   // as much of a tile's work per CTA as the tensor memory holds: fewer CTAs
   // read the same planes
@@ -1636,22 +1637,25 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   if (a.nmb * a.nsy * ncn > 512) return 1;
   int ncols = 32;
   while (ncols < a.nmb * a.nsy * ncn) ncols <<= 1;
-  // pads that spread the groups of neighbouring lanes over the banks
-  auto pad = [](int groups) { return groups <= 2 ? 64 : (groups <= 4 ? 32 : 16); };
-  a.gx = 18 * 8 * 16 + pad(ngi);
-  a.ga = 16 * 8 * 16 + pad(ngo);
   auto per_sm_of = [&](int na, int nring) {
-    const size_t sm = rg_smem_bytes(ngi, ngo, a.gx, a.ga, na, nring);
+    const size_t sm = rg_smem_bytes(a.ncb, a.pw, na, nring);
     if (sm > kHaloMaxSmem) return 0;
     return std::min((int)(g_smem_per_sm / (((sm + 127) / 128) * 128 + g_smem_reserved)), 512 / ncols);
   };
-  // two CTAs per SM where eight planes and three dY operands fit twice, else
-  // one; then the longest ring (four planes at least)
+  // two CTAs per SM where eight planes and three dY tiles fit twice, else one;
+  // then the longest ring (four planes at least)
   int per_sm = per_sm_of(3, 8) >= 2 ? 2 : 1;
-  a.na = per_sm_of(3, 7) >= per_sm ? 3 : 2;
+  a.na = per_sm_of(kRgMaxA, 8) >= per_sm ? kRgMaxA : (per_sm_of(3, 6) >= per_sm ? 3 : 2);
   a.nring = kRgMaxRing;
   while (a.nring > 4 && per_sm_of(a.na, a.nring) < per_sm) a.nring--;
   if (per_sm_of(a.na, a.nring) < per_sm) return 1;
+  CUtensorMap tmx, tmy;
+  if (encode_view(&tmx, a.x.p, a.x.cstride, a.x.coff, cin, nb, D, H, W, 8, kHaloY, 1, "wgrad", 16,
+                  CU_TENSOR_MAP_SWIZZLE_32B) ||
+      encode_view(&tmy, a.dy.p, a.dy.cstride, a.dy.coff, 8 * ngo, nb, D, H, W, 10, 16, 1, "wgrad", a.pw,
+                  a.pw == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
+                             : (a.pw == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B)))
+    return -1;
   a.ty = (H + 15) / 16;
   a.tx = (W + 2 + 7) / 8;
   const int njob = (3 / a.nsy) * (a.nmbt / a.nmb);
@@ -1679,6 +1683,9 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(conv_wgrad_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kHaloMaxSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(conv_wgrad_ring_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
     attr = true;
   }
@@ -1688,7 +1695,7 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   a.part = scr;
   a.bpart = db ? scr + (size_t)a.groups * n : nullptr;
   conv_wgrad_ring_kernel<<<(unsigned)(a.groups * njob), kRgThreads,
-                           rg_smem_bytes(ngi, ngo, a.gx, a.ga, a.na, a.nring), st>>>(a);
+                           rg_smem_bytes(a.ncb, a.pw, a.na, a.nring), st>>>(tmx, tmy, a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
   const long long tot = n + (db ? cout : 0);
