@@ -120,6 +120,21 @@ __device__ __forceinline__ void mma_bf16_if(uint32_t lead, uint32_t d_tmem, uint
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
+// The same, adding always, with the descriptors as 32-bit halves: a step along
+// an operand then costs one addition (a 64-bit one has two, each in line before
+// the MMA's issue)
+__device__ __forceinline__ void mma_bf16_add(uint32_t lead, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
+                                             uint32_t b_hi, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %2};\n\t"
+      "mov.b64 b, {%3, %4};\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(lead)
+      : "memory");
+}
 __device__ __forceinline__ void mma_commit_if(uint32_t lead, uint32_t mbar_smem) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"

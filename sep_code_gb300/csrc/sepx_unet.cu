@@ -1272,6 +1272,13 @@ static void launch_dep(void (*k)(P...), dim3 grid, int threads, size_t smem, voi
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);   // (errors: cudaGetLastError at the call sites)
 }
+// dw += the groups' partials of n entries, db (or NULL) += theirs of cout
+static void wg_reduce(const float *part, int groups, long long n, float *dw, const float *bpart, int cout, float *db,
+                      void *st) {
+  launch_dep(wg_reduce_kernel, (unsigned)((n + 127) / 128 + (db ? (cout + 127) / 128 : 0)), 32 * kRedSlices, 0, st, part,
+             groups, (int)n, dw, bpart, cout, db);
+}
+
 static int grid_for(long long n, int threads = 256) {
   long long g = (n + threads - 1) / threads;
   return (int)(g < 1 ? 1 : (g > 8 * 152 * 4 ? 8 * 152 * 4 : g));
@@ -1635,20 +1642,16 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   a.nsy = a.nmbt * 3 * ncn <= 512 ? 3 : 1;
   a.nmb = a.nmbt * a.nsy * ncn <= 512 ? a.nmbt : 1;
   if (a.nmb * a.nsy * ncn > 512) return 1;
-  int ncols = 32;
-  while (ncols < a.nmb * a.nsy * ncn) ncols <<= 1;
-  auto per_sm_of = [&](int na, int nring) {
-    const size_t sm = rg_smem_bytes(a.ncb, a.pw, na, nring);
-    if (sm > kHaloMaxSmem) return 0;
-    return std::min((int)(g_smem_per_sm / (((sm + 127) / 128) * 128 + g_smem_reserved)), 512 / ncols);
-  };
-  // two CTAs per SM where eight planes and three dY tiles fit twice, else one;
-  // then the longest ring (four planes at least)
-  int per_sm = per_sm_of(3, 8) >= 2 ? 2 : 1;
-  a.na = per_sm_of(kRgMaxA, 8) >= per_sm ? kRgMaxA : (per_sm_of(3, 6) >= per_sm ? 3 : 2);
+  // One CTA per SM with the longest ring that fits (four planes at least).  Two
+  // with shorter rings take 41 instead of 47 us for 16 -> 16 channels on 4 x
+  // 64^3 voxels alone, but 1155 instead of 1137 in the training step, where a
+  // data gradient's CTAs then find no room beside them and twice as many
+  // partials are added.
+  auto fits = [&](int na, int nring) { return rg_smem_bytes(a.ncb, a.pw, na, nring) <= kHaloMaxSmem; };
+  a.na = fits(kRgMaxA, 8) ? kRgMaxA : (fits(3, 6) ? 3 : 2);
   a.nring = kRgMaxRing;
-  while (a.nring > 4 && per_sm_of(a.na, a.nring) < per_sm) a.nring--;
-  if (per_sm_of(a.na, a.nring) < per_sm) return 1;
+  while (a.nring > 4 && !fits(a.na, a.nring)) a.nring--;
+  if (!fits(a.na, a.nring)) return 1;
   CUtensorMap tmx, tmy;
   if (encode_view(&tmx, a.x.p, a.x.cstride, a.x.coff, cin, nb, D, H, W, 8, kHaloY, 1, "wgrad", 16,
                   CU_TENSOR_MAP_SWIZZLE_32B) ||
@@ -1659,7 +1662,7 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   a.ty = (H + 15) / 16;
   a.tx = (W + 2 + 7) / 8;
   const int njob = (3 / a.nsy) * (a.nmbt / a.nmb);
-  const int slots = std::max(1, g_num_sms * per_sm / njob);
+  const int slots = std::max(1, g_num_sms / njob);
   // planes per window: the run with the least work on the busiest CTA (a
   // window loads two planes more than it has tiles; counted half a tile each)
   const long long cols = (long long)nb * a.ty * a.tx;
@@ -1679,28 +1682,31 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   a.nitems = (int)(cols * a.nzc);
   a.groups = std::min(a.nitems, slots);
   a.err = err;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(conv_wgrad_ring_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kHaloMaxSmem);
+  // 16, 32, 64 rows' channels x (three sy stacked, one sy stacked, one sy per dz)
+  const decltype(&conv_wgrad_ring_kernel<16, 3, true>) kerns[9] = {
+      conv_wgrad_ring_kernel<16, 3, true>, conv_wgrad_ring_kernel<16, 1, true>, conv_wgrad_ring_kernel<16, 1, false>,
+      conv_wgrad_ring_kernel<32, 3, true>, conv_wgrad_ring_kernel<32, 1, true>, conv_wgrad_ring_kernel<32, 1, false>,
+      conv_wgrad_ring_kernel<64, 3, true>, conv_wgrad_ring_kernel<64, 1, true>, conv_wgrad_ring_kernel<64, 1, false>};
+  const int ki = 3 * (a.pw >> 5) + (a.nsy == 3 ? 0 : (a.stacked ? 1 : 2));   // three sy fit only where stacked does
+  const auto kern = kerns[ki];
+  static bool attr[9] = {};
+  if (!attr[ki]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHaloMaxSmem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(conv_wgrad_ring_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
-    attr = true;
+    attr[ki] = true;
   }
   const long long n = 27LL * cin * cout;
   float *scr;
   if (unet_scratch(kScrGrad, (size_t)a.groups * (size_t)(n + cout), &scr, st)) return -1;
   a.part = scr;
   a.bpart = db ? scr + (size_t)a.groups * n : nullptr;
-  conv_wgrad_ring_kernel<<<(unsigned)(a.groups * njob), kRgThreads,
-                           rg_smem_bytes(a.ncb, a.pw, a.na, a.nring), st>>>(tmx, tmy, a);
+  kern<<<(unsigned)(a.groups * njob), kRgThreads, rg_smem_bytes(a.ncb, a.pw, a.na, a.nring), st>>>(tmx, tmy, a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
-  const long long tot = n + (db ? cout : 0);
-  launch_dep(wg_reduce_kernel, (unsigned)((tot + 31) / 32), 32 * kRedSlices, 0, st, a.part, a.groups, n, dw, a.bpart,
-             db ? cout : 0, db);
+  wg_reduce(a.part, a.groups, n, dw, a.bpart, cout, db, st);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet wgrad: %s", cudaGetErrorString(e));
 }
@@ -1780,9 +1786,7 @@ int conv_wgrad_tma(const void *x, int x_cstride, int x_coff, int nb, int D, int 
   conv_wgrad_tma_kernel<<<(unsigned)(a.groups * nzg), kWgThreads, smem, st>>>(tmx, tmy, a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
-  const long long tot = n + cout;
-  launch_dep(wg_reduce_kernel, (unsigned)((tot + 31) / 32), 32 * kRedSlices, 0, st, a.part, a.groups, n, dw, a.bpart,
-             cout, db);
+  wg_reduce(a.part, a.groups, n, dw, a.bpart, cout, db, st);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet wgrad: %s", cudaGetErrorString(e));
 }
@@ -2007,7 +2011,7 @@ int sepx_unet_conv_wgrad_bias(const void *x, int x_cstride, int x_coff, int nb, 
     float *bscr = scr + (size_t)blocks * 16;
     wgrad1x1_kernel<16, 1><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(xv, dv, V, scr, bscr);
     // the same fixed-order sum as the tap-stacked kernels
-    launch_dep(wg_reduce_kernel, 1, 32 * kRedSlices, 0, stream, scr, (int)blocks, 16, dw, bscr, 1, db);
+    wg_reduce(scr, (int)blocks, 16, dw, bscr, 1, db, stream);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : set_error("unet wgrad: %s", cudaGetErrorString(e));
   }
@@ -2044,8 +2048,7 @@ int sepx_unet_conv_wgrad_bias(const void *x, int x_cstride, int x_coff, int nb, 
       xv, nb, D, H, W, cin, ntap, dv, cout, np, (int)per, dw, err, part);
   if (part) {
     const long long n = mtot * cout;
-    launch_dep(wg_reduce_kernel, (unsigned)((n + 31) / 32), 32 * kRedSlices, 0, stream, part, (int)splits, n, dw,
-               nullptr, 0, nullptr);
+    wg_reduce(part, (int)splits, n, dw, nullptr, 0, nullptr, stream);
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet wgrad: %s", cudaGetErrorString(e));
