@@ -883,7 +883,7 @@ __global__ void __launch_bounds__(256, 3) conv1x1_kernel(View x, long long V, co
                                                       const float *bias, int relu, __nv_bfloat16 *y,
                                                       int y_cstride, int y_coff, float *yf,
                                                       const float *resid, View mask) {
-  __shared__ float w[COUT][CIN];
+  __shared__ __align__(16) float w[COUT][CIN];
   __shared__ float bs[COUT];
   for (int i = threadIdx.x; i < COUT * CIN; i += blockDim.x) {
     const int n = i / CIN, k = i % CIN;
@@ -891,44 +891,63 @@ __global__ void __launch_bounds__(256, 3) conv1x1_kernel(View x, long long V, co
   }
   for (int i = threadIdx.x; i < COUT; i += blockDim.x) bs[i] = bias ? bias[i] : 0.f;
   __syncthreads();
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V;
-       v += (long long)gridDim.x * blockDim.x) {
-    float xin[CIN];
+  // NV voxels per thread and pass: the weights, read again from shared memory
+  // (in registers they cost a memory-bound kernel its warps), bound the kernel
+  // with one (16 outputs, 4 x 64^3 voxels: 28.6 us, 23.9 with two)
+  constexpr int NV = COUT > 1 ? 2 : 1;
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long v0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; v0 < V; v0 += NV * step) {
+    float xin[NV][CIN];
 #pragma unroll
-    for (int g = 0; g < CIN / 8; g++) {
-      const uint4 q = *reinterpret_cast<const uint4 *>(x.p + v * x.cstride + x.coff + 8 * g);
-      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&q);
+    for (int j = 0; j < NV; j++) {
+      const long long v = v0 + j * step < V ? v0 + j * step : v0;
 #pragma unroll
-      for (int i = 0; i < 8; i++) xin[8 * g + i] = __bfloat162float(h[i]);
-    }
-    float acc[COUT];
-    // weights re-read from shared memory per voxel (broadcast loads), not
-    // held in registers: a memory-bound kernel needs its warps more
-    const volatile float(*wv)[CIN] = w;
+      for (int g = 0; g < CIN / 8; g++) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(x.p + v * x.cstride + x.coff + 8 * g);
+        const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&q);
 #pragma unroll
-    for (int n = 0; n < COUT; n++) {
-      float t = 0.f;
-#pragma unroll
-      for (int k = 0; k < CIN; k++) t = __fmaf_rn(wv[n][k], xin[k], t);
-      t += bs[n];
-      acc[n] = relu ? fmaxf(t, 0.f) : t;
-    }
-    if (mask.p) {
-#pragma unroll
-      for (int g = 0; g < COUT / 8; g++) mask8(mask.p + v * mask.cstride + mask.coff + 8 * g, acc + 8 * g);
-    }
-    if (y) {
-#pragma unroll
-      for (int g = 0; g < COUT / 8; g++) {
-        __align__(16) __nv_bfloat16 h[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) h[i] = __float2bfloat16_rn(acc[8 * g + i]);
-        *reinterpret_cast<uint4 *>(y + v * y_cstride + y_coff + 8 * g) = *reinterpret_cast<const uint4 *>(h);
+        for (int i = 0; i < 8; i++) xin[j][8 * g + i] = __bfloat162float(h[i]);
       }
     }
-    if (yf) {
+    constexpr int NG = COUT < 8 ? COUT : 8;   // outputs of a pass over the weights
 #pragma unroll
-      for (int n = 0; n < COUT; n++) yf[v * COUT + n] = acc[n] + (resid ? resid[v * COUT + n] : 0.f);
+    for (int n0 = 0; n0 < COUT; n0 += NG) {
+      float acc[NV][NG];
+#pragma unroll
+      for (int n = 0; n < NG; n++) {
+        float t[NV];
+#pragma unroll
+        for (int j = 0; j < NV; j++) t[j] = 0.f;
+#pragma unroll
+        for (int k = 0; k < CIN; k += 4) {
+          const float4 q = lds4(&w[n0 + n][k]);
+#pragma unroll
+          for (int j = 0; j < NV; j++) {
+            t[j] = __fmaf_rn(q.x, xin[j][k], t[j]);
+            t[j] = __fmaf_rn(q.y, xin[j][k + 1], t[j]);
+            t[j] = __fmaf_rn(q.z, xin[j][k + 2], t[j]);
+            t[j] = __fmaf_rn(q.w, xin[j][k + 3], t[j]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < NV; j++) {
+          t[j] += bs[n0 + n];
+          acc[j][n] = relu ? fmaxf(t[j], 0.f) : t[j];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < NV; j++) {
+        const long long v = v0 + j * step;
+        if (v >= V) break;
+        if constexpr (NG == 8) {
+          if (mask.p) mask8(mask.p + v * mask.cstride + mask.coff + n0, acc[j]);
+          if (y) *reinterpret_cast<uint4 *>(y + v * y_cstride + y_coff + n0) = pack8(acc[j]);
+        }
+        if (yf) {
+#pragma unroll
+          for (int n = 0; n < NG; n++) yf[v * COUT + n0 + n] = acc[j][n] + (resid ? resid[v * COUT + n0 + n] : 0.f);
+        }
+      }
     }
   }
 }
@@ -982,141 +1001,191 @@ __global__ void __launch_bounds__(256) wgrad1x1_kernel(View x, View dy, long lon
 // ---------------------------------------------------------------------------
 // Memory-bound pieces.
 // ---------------------------------------------------------------------------
-// 2x2x2 average pooling: out (D/2, H/2, W/2)
-// element e of a walk over (voxel, 8-channel group) of an nb x D x H x W
-// volume -> group g, voxel v and its coordinates.  32-bit divisions where the
-// walk is shorter than 2^31 (every U-Net volume): several times cheaper than
-// the 64-bit ones, and these kernels are otherwise bound by them.
-struct EV {
-  long long v;
-  int g, n, z, y, x;
+// A thread takes one coarse voxel (of the pooled or not yet upsampled volume)
+// and a group of 8 channels, and walks its eight children: their loads are in
+// flight together, the coarse voxel is read or written once, and the
+// coordinates are worked out once for all eight, by multiplication with the
+// divisors' reciprocals where the walk is shorter than 2^31 elements (every
+// U-Net volume), else by 64-bit division.  Bound by memory: a slice of 16 of
+// 48 channels moves the 64-byte sectors around it too (pooling 128^3 voxels 32
+// us, as one child per thread).  Upsampling took 34.6 us there with a thread
+// per child, bound by the divisions, and takes 23 so; inference of the default
+// network at 128^3 559 -> 543.  (32-byte accesses per thread: no gain, the two
+// groups of a sector lie in neighbouring lanes.)
+struct FastDiv {
+  uint32_t m;
+  int sh;
 };
-template <typename I>
-__device__ __forceinline__ EV decode_ev_t(I e, int cg, int D, int H, int W) {
-  EV r;
-  const I v = e / (I)cg;
-  r.g = (int)(e - v * (I)cg);
-  const I q1 = v / (I)W;
-  r.x = (int)(v - q1 * (I)W);
-  const I q2 = q1 / (I)H;
-  r.y = (int)(q1 - q2 * (I)H);
-  const I q3 = q2 / (I)D;
-  r.z = (int)(q2 - q3 * (I)D);
-  r.n = (int)q3;
-  r.v = (long long)v;
+// n / d == (n * m) >> sh for n < 2^31: m = ceil(2^sh / d) with sh = 31 +
+// ceil(log2 d), so m < 2^32 and the error n (m d - 2^sh) / (d 2^sh) < 1 / d
+inline FastDiv fast_div(int d) {
+  FastDiv f;
+  int l = 0;
+  while ((1LL << l) < d) l++;
+  f.sh = 31 + l;
+  f.m = (uint32_t)((((unsigned long long)1 << f.sh) + (unsigned long long)d - 1) / (unsigned long long)d);
+  return f;
+}
+__device__ __forceinline__ uint32_t operator/(uint32_t n, FastDiv f) {
+  return (uint32_t)(((unsigned long long)n * f.m) >> f.sh);
+}
+// the walk over (voxel, group): nb x D x H x W voxels (coarse ones, but for avgpool_bwd)
+struct Walk {
+  int D, H, W, cu;          // cu: groups per voxel
+  long long total;
+  FastDiv dc, dw, dh, dd;
+};
+inline Walk make_walk(int nb, int D, int H, int W, int cu) {
+  return Walk{D, H, W, cu, (long long)nb * D * H * W * cu, fast_div(std::max(cu, 1)), fast_div(W), fast_div(H), fast_div(D)};
+}
+// element e -> group, voxel and its coordinates
+struct Elem {
+  int u, x, y, z;
+  long long v, n;
+};
+__device__ __forceinline__ Elem walk_elem(const Walk &w, long long e) {
+  Elem r;
+  if (w.total < (1LL << 31)) {
+    const uint32_t v = (uint32_t)e / w.dc, q1 = v / w.dw, q2 = q1 / w.dh, q3 = q2 / w.dd;
+    r.u = (int)((uint32_t)e - v * (uint32_t)w.cu);
+    r.x = (int)(v - q1 * (uint32_t)w.W);
+    r.y = (int)(q1 - q2 * (uint32_t)w.H);
+    r.z = (int)(q2 - q3 * (uint32_t)w.D);
+    r.n = q3;
+    r.v = v;
+  } else {
+    r.v = e / w.cu;
+    r.u = (int)(e - r.v * w.cu);
+    const long long q1 = r.v / w.W, q2 = q1 / w.H;
+    r.x = (int)(r.v - q1 * w.W);
+    r.y = (int)(q1 - q2 * w.H);
+    r.n = q2 / w.D;
+    r.z = (int)(q2 - r.n * w.D);
+  }
   return r;
 }
-__device__ __forceinline__ EV decode_ev(long long e, bool narrow, int cg, int D, int H, int W) {
-  return narrow ? decode_ev_t<uint32_t>((uint32_t)e, cg, D, H, W) : decode_ev_t<long long>(e, cg, D, H, W);
+// the first child's voxel index
+__device__ __forceinline__ long long first_child(const Walk &w, const Elem &c) {
+  return (((c.n * 2 * w.D + 2 * c.z) * 2 * w.H + 2 * c.y) * 2 * w.W) + 2 * c.x;
+}
+// voxel offset of child k = 4 dz + 2 dy + dx from the first
+__device__ __forceinline__ long long child_off(const Walk &w, int k) {
+  return (k >> 2) * (4LL * w.H * w.W) + ((k >> 1) & 1) * (2LL * w.W) + (k & 1);
 }
 
-__global__ void avgpool_kernel(View x, int nb, int D, int H, int W, int c, __nv_bfloat16 *y,
-                               int y_cstride, int y_coff) {
-  const int D2 = D / 2, H2 = H / 2, W2 = W / 2, cg = c / 8;
-  const long long total = (long long)nb * D2 * H2 * W2 * cg;
-  const bool narrow = total < (1LL << 31);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const EV c4 = decode_ev(e, narrow, cg, D2, H2, W2);
-    const int g = c4.g, xx = c4.x, yy = c4.y, zz = c4.z, n = c4.n;
-    const long long v = c4.v;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int d = 0; d < 8; d++) {
-      const long long vi = (((long long)n * D + 2 * zz + (d >> 2)) * H + 2 * yy + ((d >> 1) & 1)) * W +
-                           2 * xx + (d & 1);
-      const uint4 q = *reinterpret_cast<const uint4 *>(x.p + vi * x.cstride + x.coff + g * 8);
-      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&q);
+// 8 channels of a voxel
+struct Ch {
+  uint32_t r[4];
+  __device__ __forceinline__ void load(const __nv_bfloat16 *p) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(p);
+    r[0] = q.x; r[1] = q.y; r[2] = q.z; r[3] = q.w;
+  }
+  __device__ __forceinline__ void store(__nv_bfloat16 *p) const {
+    *reinterpret_cast<uint4 *>(p) = make_uint4(r[0], r[1], r[2], r[3]);
+  }
+  __device__ __forceinline__ float lo(int i) const { return __uint_as_float(r[i] << 16); }
+  __device__ __forceinline__ float hi(int i) const { return __uint_as_float(r[i] & 0xffff0000u); }
+  __device__ __forceinline__ void set(int i, float l, float h) {
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r[i]) : "f"(h), "f"(l));
+  }
+  // ReLU backward: zero where the activation m is not > 0
+  __device__ __forceinline__ void relu(const Ch &m) {
 #pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] += __bfloat162float(h[i]);
+    for (int i = 0; i < 4; i++) {
+      if (!(m.lo(i) > 0.f)) r[i] &= 0xffff0000u;
+      if (!(m.hi(i) > 0.f)) r[i] &= 0xffffu;
     }
-    __align__(16) __nv_bfloat16 o[8];
+  }
+};
+
+// the eight children's sums in child order, four children's loads in flight
+__device__ __forceinline__ void sum_children(const __nv_bfloat16 *src, int cstride, const Walk &w, float (&a)[8]) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) o[i] = __float2bfloat16_rn(acc[i] * 0.125f);
-    *reinterpret_cast<uint4 *>(y + v * y_cstride + y_coff + g * 8) = *reinterpret_cast<const uint4 *>(o);
+  for (int i = 0; i < 8; i++) a[i] = 0.f;
+#pragma unroll
+  for (int h = 0; h < 8; h += 4) {
+    Ch q[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) q[k].load(src + child_off(w, h + k) * cstride);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        a[2 * i] += q[k].lo(i);
+        a[2 * i + 1] += q[k].hi(i);
+      }
   }
 }
 
-// gradient of avgpool: dx (D, H, W) = dy(parent) / 8
-__global__ void avgpool_bwd_kernel(View dy, int nb, int D, int H, int W, int c, __nv_bfloat16 *dx,
-                                   int dx_cstride, int dx_coff, int accumulate, View mask) {
-  const int D2 = D / 2, H2 = H / 2, W2 = W / 2, cg = c / 8;
-  const long long total = (long long)nb * D * H * W * cg;
-  const bool narrow = total < (1LL << 31);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+// 2x2x2 average pooling
+__global__ void __launch_bounds__(256) avgpool_kernel(View x, Walk w, __nv_bfloat16 *y, int y_cstride, int y_coff) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < w.total;
        e += (long long)gridDim.x * blockDim.x) {
-    const EV c4 = decode_ev(e, narrow, cg, D, H, W);
-    const int g = c4.g, xx = c4.x, yy = c4.y, zz = c4.z, n = c4.n;
-    const long long v = c4.v;
-    const long long vp = (((long long)n * D2 + zz / 2) * H2 + yy / 2) * W2 + xx / 2;
-    const uint4 q = *reinterpret_cast<const uint4 *>(dy.p + vp * dy.cstride + dy.coff + g * 8);
-    const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&q);
-    __nv_bfloat16 *dst = dx + v * dx_cstride + dx_coff + g * 8;
-    __align__(16) __nv_bfloat16 o[8];
-    const uint4 old = accumulate ? *reinterpret_cast<const uint4 *>(dst) : make_uint4(0, 0, 0, 0);
-    const __nv_bfloat16 *ho = reinterpret_cast<const __nv_bfloat16 *>(&old);
+    const Elem c = walk_elem(w, e);
+    const __nv_bfloat16 *src = x.p + first_child(w, c) * x.cstride + x.coff + 8 * c.u;
+    float a[8];
+    sum_children(src, x.cstride, w, a);
+    Ch o;
 #pragma unroll
-    for (int i = 0; i < 8; i++)
-      o[i] = __float2bfloat16_rn(__bfloat162float(h[i]) * 0.125f + (accumulate ? __bfloat162float(ho[i]) : 0.f));
-    if (mask.p) {   // ReLU backward of the layer whose output this is (after the sum)
-      const uint4 qm = *reinterpret_cast<const uint4 *>(mask.p + v * mask.cstride + mask.coff + g * 8);
-      const __nv_bfloat16 *hm = reinterpret_cast<const __nv_bfloat16 *>(&qm);
+    for (int i = 0; i < 4; i++) o.set(i, a[2 * i] * 0.125f, a[2 * i + 1] * 0.125f);
+    o.store(y + c.v * y_cstride + y_coff + 8 * c.u);
+  }
+}
+
+// gradient of avgpool: dx = dy(parent) / 8 (+ dx), then the ReLU backward of
+// the layer whose output this is.  w walks the children: a thread per parent
+// with its eight takes longer beside the weight gradients (a training step on
+// 4 x 64^3: 1175 us against 1146)
+__global__ void __launch_bounds__(256) avgpool_bwd_kernel(View dy, Walk w, __nv_bfloat16 *dx, int dx_cstride, int dx_coff,
+                                                          int accumulate, View mask) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < w.total;
+       e += (long long)gridDim.x * blockDim.x) {
+    const Elem c = walk_elem(w, e);
+    const long long vp = ((c.n * (w.D / 2) + c.z / 2) * (w.H / 2) + c.y / 2) * (w.W / 2) + c.x / 2;
+    __nv_bfloat16 *dst = dx + c.v * dx_cstride + dx_coff + 8 * c.u;
+    Ch d, o, m;
+    d.load(dy.p + vp * dy.cstride + dy.coff + 8 * c.u);
+    if (accumulate) o.load(dst);
+    if (mask.p) m.load(mask.p + c.v * mask.cstride + mask.coff + 8 * c.u);
 #pragma unroll
-      for (int i = 0; i < 8; i++)
-        if (!(__bfloat162float(hm[i]) > 0.f)) o[i] = __float2bfloat16_rn(0.f);
-    }
-    *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(o);
+    for (int i = 0; i < 4; i++)
+      o.set(i, d.lo(i) * 0.125f + (accumulate ? o.lo(i) : 0.f), d.hi(i) * 0.125f + (accumulate ? o.hi(i) : 0.f));
+    if (mask.p) o.relu(m);
+    o.store(dst);
   }
 }
 
 // nearest upsampling x2: out (2D, 2H, 2W)
-__global__ void upsample_kernel(View x, int nb, int D, int H, int W, int c, __nv_bfloat16 *y,
-                                int y_cstride, int y_coff) {
-  const int cg = c / 8;
-  const int D2 = 2 * D, H2 = 2 * H, W2 = 2 * W;
-  const long long total = (long long)nb * D2 * H2 * W2 * cg;
-  const bool narrow = total < (1LL << 31);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+__global__ void __launch_bounds__(256) upsample_kernel(View x, Walk w, __nv_bfloat16 *y, int y_cstride, int y_coff) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < w.total;
        e += (long long)gridDim.x * blockDim.x) {
-    const EV c4 = decode_ev(e, narrow, cg, D2, H2, W2);
-    const int g = c4.g, xx = c4.x, yy = c4.y, zz = c4.z, n = c4.n;
-    const long long v = c4.v;
-    const long long vs = (((long long)n * D + zz / 2) * H + yy / 2) * W + xx / 2;
-    *reinterpret_cast<uint4 *>(y + v * y_cstride + y_coff + g * 8) =
-        *reinterpret_cast<const uint4 *>(x.p + vs * x.cstride + x.coff + g * 8);
+    const Elem c = walk_elem(w, e);
+    Ch q;
+    q.load(x.p + c.v * x.cstride + x.coff + 8 * c.u);
+    __nv_bfloat16 *dst = y + first_child(w, c) * y_cstride + y_coff + 8 * c.u;
+#pragma unroll
+    for (int k = 0; k < 8; k++) q.store(dst + child_off(w, k) * y_cstride);
   }
 }
 
-// gradient of upsampling: dx (D, H, W) = sum of the 8 children
-__global__ void upsample_bwd_kernel(View dy, int nb, int D, int H, int W, int c, __nv_bfloat16 *dx,
-                                    int dx_cstride, int dx_coff, View mask) {
-  const int cg = c / 8;
-  const long long total = (long long)nb * D * H * W * cg;
-  const bool narrow = total < (1LL << 31);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+// gradient of upsampling: dx = sum of the 8 children, then the ReLU backward
+__global__ void __launch_bounds__(256) upsample_bwd_kernel(View dy, Walk w, __nv_bfloat16 *dx, int dx_cstride,
+                                                           int dx_coff, View mask) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < w.total;
        e += (long long)gridDim.x * blockDim.x) {
-    const EV c4 = decode_ev(e, narrow, cg, D, H, W);
-    const int g = c4.g, xx = c4.x, yy = c4.y, zz = c4.z, n = c4.n;
-    const long long v = c4.v;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int d = 0; d < 8; d++) {
-      const long long vc = (((long long)n * 2 * D + 2 * zz + (d >> 2)) * 2 * H + 2 * yy + ((d >> 1) & 1)) *
-                               2 * W + 2 * xx + (d & 1);
-      const uint4 q = *reinterpret_cast<const uint4 *>(dy.p + vc * dy.cstride + dy.coff + g * 8);
-      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&q);
+    const Elem c = walk_elem(w, e);
+    const __nv_bfloat16 *src = dy.p + first_child(w, c) * dy.cstride + dy.coff + 8 * c.u;
+    float a[8];
+    sum_children(src, dy.cstride, w, a);
+    Ch o;
 #pragma unroll
-      for (int i = 0; i < 8; i++) acc[i] += __bfloat162float(h[i]);
-    }
-    __align__(16) __nv_bfloat16 o[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) o[i] = __float2bfloat16_rn(acc[i]);
+    for (int i = 0; i < 4; i++) o.set(i, a[2 * i], a[2 * i + 1]);
     if (mask.p) {
-      const uint4 qm = *reinterpret_cast<const uint4 *>(mask.p + v * mask.cstride + mask.coff + g * 8);
-      const __nv_bfloat16 *hm = reinterpret_cast<const __nv_bfloat16 *>(&qm);
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-        if (!(__bfloat162float(hm[i]) > 0.f)) o[i] = __float2bfloat16_rn(0.f);
+      Ch m;
+      m.load(mask.p + c.v * mask.cstride + mask.coff + 8 * c.u);
+      o.relu(m);
     }
-    *reinterpret_cast<uint4 *>(dx + v * dx_cstride + dx_coff + g * 8) = *reinterpret_cast<const uint4 *>(o);
+    o.store(dx + c.v * dx_cstride + dx_coff + 8 * c.u);
   }
 }
 
@@ -1236,7 +1305,11 @@ __global__ void adam_kernel(float *p, const float *g, float *m, float *v, long l
     }
     step = (int)s;
   }
-  const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
+  // one thread per block forms them (every thread: 12.6 us for 681 k parameters, 10.9 so)
+  __shared__ float corr[2];
+  if (threadIdx.x < 2) corr[threadIdx.x] = 1.f - powf(threadIdx.x ? b2 : b1, (float)step);
+  __syncthreads();
+  const float c1 = corr[0], c2 = corr[1];
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     const float gi = g[i];
@@ -2060,8 +2133,9 @@ int sepx_unet_avgpool(const void *x, int x_cstride, int x_coff, int nb, int D, i
     return -1;
   if (c % 8 || D % 2 || H % 2 || W % 2) return set_error("unet avgpool: bad shape");
   View xv{(const __nv_bfloat16 *)x, x_cstride, x_coff};
-  avgpool_kernel<<<grid_for((long long)nb * D * H * W / 8 * (c / 8)), 256, 0, (cudaStream_t)stream>>>(
-      xv, nb, D, H, W, c, (__nv_bfloat16 *)y, y_cstride, y_coff);
+  const Walk w = make_walk(nb, D / 2, H / 2, W / 2, c / 8);
+  avgpool_kernel<<<grid_for(w.total), 256, 0, (cudaStream_t)stream>>>(
+      xv, w, (__nv_bfloat16 *)y, y_cstride, y_coff);
   return cudaGetLastError() == cudaSuccess ? 0 : set_error("unet avgpool: launch failed");
 }
 
@@ -2082,8 +2156,9 @@ int sepx_unet_avgpool_bwd_masked(const void *dy, int dy_cstride, int dy_coff, in
     return set_error("unet avgpool_bwd: bad mask view");
   View dv{(const __nv_bfloat16 *)dy, dy_cstride, dy_coff};
   View mv{(const __nv_bfloat16 *)mask, mask_cstride, mask_coff};
-  avgpool_bwd_kernel<<<grid_for((long long)nb * D * H * W * (c / 8)), 256, 0, (cudaStream_t)stream>>>(
-      dv, nb, D, H, W, c, (__nv_bfloat16 *)dx, dx_cstride, dx_coff, accumulate, mv);
+  const Walk w = make_walk(nb, D, H, W, c / 8);
+  avgpool_bwd_kernel<<<grid_for(w.total), 256, 0, (cudaStream_t)stream>>>(
+      dv, w, (__nv_bfloat16 *)dx, dx_cstride, dx_coff, accumulate, mv);
   return cudaGetLastError() == cudaSuccess ? 0 : set_error("unet avgpool_bwd: launch failed");
 }
 
@@ -2093,8 +2168,9 @@ int sepx_unet_upsample(const void *x, int x_cstride, int x_coff, int nb, int D, 
     return -1;
   if (c % 8) return set_error("unet upsample: bad shape");
   View xv{(const __nv_bfloat16 *)x, x_cstride, x_coff};
-  upsample_kernel<<<grid_for((long long)nb * D * H * W * 8 * (c / 8)), 256, 0, (cudaStream_t)stream>>>(
-      xv, nb, D, H, W, c, (__nv_bfloat16 *)y, y_cstride, y_coff);
+  const Walk w = make_walk(nb, D, H, W, c / 8);
+  upsample_kernel<<<grid_for(w.total), 256, 0, (cudaStream_t)stream>>>(
+      xv, w, (__nv_bfloat16 *)y, y_cstride, y_coff);
   return cudaGetLastError() == cudaSuccess ? 0 : set_error("unet upsample: launch failed");
 }
 
@@ -2115,8 +2191,9 @@ int sepx_unet_upsample_bwd_masked(const void *dy, int dy_cstride, int dy_coff, i
     return set_error("unet upsample_bwd: bad mask view");
   View dv{(const __nv_bfloat16 *)dy, dy_cstride, dy_coff};
   View mv{(const __nv_bfloat16 *)mask, mask_cstride, mask_coff};
-  upsample_bwd_kernel<<<grid_for((long long)nb * D * H * W * (c / 8)), 256, 0, (cudaStream_t)stream>>>(
-      dv, nb, D, H, W, c, (__nv_bfloat16 *)dx, dx_cstride, dx_coff, mv);
+  const Walk w = make_walk(nb, D, H, W, c / 8);
+  upsample_bwd_kernel<<<grid_for(w.total), 256, 0, (cudaStream_t)stream>>>(
+      dv, w, (__nv_bfloat16 *)dx, dx_cstride, dx_coff, mv);
   return cudaGetLastError() == cudaSuccess ? 0 : set_error("unet upsample_bwd: launch failed");
 }
 
