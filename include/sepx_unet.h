@@ -61,6 +61,12 @@ int sepx_unet_set_halo(int enable);
  * kernel; 1 the per-tile kernel, else gather; 0 gather.  Returns the
  * previous choice, or -1 for another value. */
 int sepx_unet_set_wgrad_form(int form);
+/* The BF16 convolution and the 2x2x2 average of its output into the view p
+ * (D, H, W even): the same bits as sepx_unet_conv_fwd, then sepx_unet_avgpool,
+ * in one pass on the z-walk kernel, else as these two. */
+int sepx_unet_conv_fwd_pool(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
+                            int ntap, const void *wpacked, const float *bias, int cout, int relu, void *y,
+                            int y_cstride, int y_coff, void *p, int p_cstride, int p_coff, void *stream);
 /* dw[t*cin + c][cout] += sum_v x[v + off(t)][c] dy[v][cout]  (FP32
  * accumulation); dy holds cout rounded up to 8 channels at dy_coff */
 int sepx_unet_conv_wgrad(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W,

@@ -1536,14 +1536,20 @@ int conv_halo(const void *x, int x_cstride, int x_coff, int nb, int D, int H, in
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
 }
 
+struct PoolOut {
+  __nv_bfloat16 *p;
+  int cstride, coff;
+};
+
 // The z-walk convolution (sepx_unet_zwfwd.inc): every layer the halo-staged
 // kernel takes whose three column blocks fit one MMA (3 x np <= 256; it
 // measured 2.4 to 5.1 times as fast on those).  Returns 1 where it does not
 // apply (np >= 96: the halo-staged kernel).
 int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
                const void *wpacked, const float *bias, int cout, int np, int relu, void *y, int y_cstride,
-               int y_coff, float *yf, const float *resid, View mask, int *err, cudaStream_t st) {
+               int y_coff, float *yf, const float *resid, View mask, int *err, const PoolOut *pool, cudaStream_t st) {
   if (3 * np > 256) return 1;
+  if (pool && (D % 2 || H % 2 || W % 2)) return 1;
   if (unet_dev_init()) return -1;
   auto fit = [&](int nslot) {
     const size_t sm = zf_smem_bytes(cin, np, nslot);
@@ -1561,6 +1567,9 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.np = np; a.relu = relu;
   a.bias = bias; a.y = (__nv_bfloat16 *)y; a.y_cstride = y_cstride; a.y_coff = y_coff;
   a.yf = yf; a.resid = resid; a.err = err; a.mask = mask;
+  a.pool = pool ? pool->p : nullptr;
+  a.pool_cstride = pool ? pool->cstride : 0;
+  a.pool_coff = pool ? pool->coff : 0;
   a.nslot = kZfMinSlots;
   while (a.nslot < kZfMaxSlots && fit(a.nslot + 1) >= per_sm) a.nslot++;
   a.ty = (H + kTileY - 1) / kTileY;
@@ -1576,7 +1585,8 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   const int zmax = std::min(std::min(kZfMaxZ, D), (512 / per_sm) / np);
   double best = 1e300;
   a.zc = 1;
-  for (int zc = 1; zc <= zmax; zc++) {
+  const int zstep = pool ? 2 : 1;   // (pooled: windows of whole plane pairs)
+  for (int zc = zstep; zc <= zmax; zc += zstep) {
     const long long items = cols * ((D + zc - 1) / zc);
     const long long per = (items + slots - 1) / slots;
     double c = 0;
@@ -1591,19 +1601,23 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   }
   a.nzc = (D + a.zc - 1) / a.zc;
   a.zc = (D + a.nzc - 1) / a.nzc;   // the same windows, evenly filled
+  if (pool) {
+    a.zc += a.zc & 1;
+    a.nzc = (D + a.zc - 1) / a.zc;
+  }
   a.nitems = (int)(cols * a.nzc);
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(conv_zwalk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kHaloMaxSmem);
+  const auto kern = pool ? conv_zwalk_kernel<true> : conv_zwalk_kernel<false>;
+  static bool attr[2] = {};
+  if (!attr[pool != nullptr]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHaloMaxSmem);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(conv_zwalk_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return set_error("unet conv: %s", cudaGetErrorString(e));
-    attr = true;
+    attr[pool != nullptr] = true;
   }
   const long long grid = std::min<long long>(a.nitems, slots);
-  launch_dep(conv_zwalk_kernel, (unsigned)grid, kZfThreads, zf_smem_bytes(cin, np, a.nslot), st, tm,
+  launch_dep(kern, (unsigned)grid, kZfThreads, zf_smem_bytes(cin, np, a.nslot), st, tm,
              (const __nv_bfloat16 *)wpacked, a);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
@@ -1948,17 +1962,12 @@ int sepx_unet_pack_weights_many(int njobs, const float *const *w, void *const *o
   return e == cudaSuccess ? 0 : set_error("unet pack: %s", cudaGetErrorString(e));
 }
 
-int sepx_unet_conv_fwd(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
-                       int ntap, const void *wpacked, const float *bias, int cout, int relu, void *y,
-                       int y_cstride, int y_coff, float *yf, const float *resid, void *stream) {
-  return sepx_unet_conv_fwd_masked(x, x_cstride, x_coff, nb, D, H, W, cin, ntap, wpacked, bias, cout, relu, y,
-                                   y_cstride, y_coff, yf, resid, nullptr, 0, 0, stream);
-}
-
-int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W,
-                              int cin, int ntap, const void *wpacked, const float *bias, int cout, int relu,
-                              void *y, int y_cstride, int y_coff, float *yf, const float *resid,
-                              const void *mask, int mask_cstride, int mask_coff, void *stream) {
+namespace {
+// the checked convolution; pool (or NULL): also y's 2x2x2 average, *pooled = 1 where it was written
+int conv_any(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin, int ntap,
+             const void *wpacked, const float *bias, int cout, int relu, void *y, int y_cstride, int y_coff, float *yf,
+             const float *resid, const void *mask, int mask_cstride, int mask_coff, const PoolOut *pool, int *pooled,
+             void *stream) {
   if (need_dev(x, "conv x") || need_dev(wpacked, "conv weights") || need_dims(nb, D, H, W, "conv"))
     return -1;
   if (mask && (cout % 8 || mask_cstride % 8 || mask_coff % 8 || mask_coff + cout > mask_cstride))
@@ -1984,8 +1993,15 @@ int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, 
     const int ngc = cin / 8;
     const uint32_t wbytes = (uint32_t)((27 * ngc + (ngc & 1)) * (np / 8) * 128);
     if (halo_smem_bytes(cin, wbytes, 1) <= kHaloMaxSmem) {
-      const int rc = conv_zwalk(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y,
-                                y_cstride, y_coff, yf, resid, mv, err, (cudaStream_t)stream);
+      int rc = 1;
+      if (pool) {
+        rc = conv_zwalk(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y, y_cstride, y_coff, yf,
+                        resid, mv, err, pool, (cudaStream_t)stream);
+        if (!rc) *pooled = 1;
+      }
+      if (rc > 0)
+        rc = conv_zwalk(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y, y_cstride, y_coff, yf,
+                        resid, mv, err, nullptr, (cudaStream_t)stream);
       if (rc <= 0) return rc;
       return conv_halo(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, wbytes, bias, cout, np, relu, y,
                        y_cstride, y_coff, yf, resid, mv, err, (cudaStream_t)stream);
@@ -2042,6 +2058,38 @@ int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, 
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
+}
+
+}  // namespace
+
+int sepx_unet_conv_fwd(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
+                       int ntap, const void *wpacked, const float *bias, int cout, int relu, void *y,
+                       int y_cstride, int y_coff, float *yf, const float *resid, void *stream) {
+  return sepx_unet_conv_fwd_masked(x, x_cstride, x_coff, nb, D, H, W, cin, ntap, wpacked, bias, cout, relu, y,
+                                   y_cstride, y_coff, yf, resid, nullptr, 0, 0, stream);
+}
+
+int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W,
+                              int cin, int ntap, const void *wpacked, const float *bias, int cout, int relu,
+                              void *y, int y_cstride, int y_coff, float *yf, const float *resid,
+                              const void *mask, int mask_cstride, int mask_coff, void *stream) {
+  return conv_any(x, x_cstride, x_coff, nb, D, H, W, cin, ntap, wpacked, bias, cout, relu, y, y_cstride, y_coff, yf,
+                  resid, mask, mask_cstride, mask_coff, nullptr, nullptr, stream);
+}
+
+int sepx_unet_conv_fwd_pool(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
+                            int ntap, const void *wpacked, const float *bias, int cout, int relu, void *y,
+                            int y_cstride, int y_coff, void *p, int p_cstride, int p_coff, void *stream) {
+  if (need_dev(y, "conv y") || need_dev(p, "conv pooled y") || need_dims(nb, D, H, W, "conv")) return -1;
+  if (cout % 8 || D % 2 || H % 2 || W % 2) return set_error("unet conv_fwd_pool: bad shape");
+  if (p_cstride % 8 || p_coff % 8 || p_coff < 0 || p_coff + cout > p_cstride)
+    return set_error("unet conv_fwd_pool: bad pooled view");
+  const PoolOut pool{(__nv_bfloat16 *)p, p_cstride, p_coff};
+  int pooled = 0;
+  if (conv_any(x, x_cstride, x_coff, nb, D, H, W, cin, ntap, wpacked, bias, cout, relu, y, y_cstride, y_coff, nullptr,
+               nullptr, nullptr, 0, 0, &pool, &pooled, stream))
+    return -1;
+  return pooled ? 0 : sepx_unet_avgpool(y, y_cstride, y_coff, nb, D, H, W, cout, p, p_cstride, p_coff, stream);
 }
 
 int sepx_unet_conv_wgrad(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W,

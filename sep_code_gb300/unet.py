@@ -42,6 +42,7 @@ _SIGS = {
                            _vp, _vp],
     "sepx_unet_conv_fwd_masked": [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i, _i,
                                   _vp, _vp, _vp, _i, _i, _vp],
+    "sepx_unet_conv_fwd_pool": [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _i, _vp, _i, _i, _vp, _i, _i, _vp],
     "sepx_unet_conv_wgrad": [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp],
     "sepx_unet_conv_wgrad_bias": [_vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _i, _i, _i, _vp, _vp, _vp],
     "sepx_unet_avgpool": [_vp, _i, _i, _i, _i, _i, _i, _i, _vp, _i, _i, _vp],
@@ -255,6 +256,14 @@ class UNet3D:
                                     _p(yf) if yf is not None else None,
                                     _p(resid) if resid is not None else None, self.stream_ptr))
 
+    def _conv_pool(self, L, x, xcs, xco, lvl, y, ycs, yco, p, pcs, pco):
+        """the convolution and the 2x2x2 average of its output"""
+        nb = self.shape[0]
+        D, H, W = self.dims[lvl]
+        _chk(lib.sepx_unet_conv_fwd_pool(_p(x), xcs, xco, nb, D, H, W, L.cin_p, L.ntap, _p(self.pk[L.name]),
+                                         _p(self.b[L.name]), L.cout, 1 if L.relu else 0, _p(y), ycs, yco,
+                                         _p(p), pcs, pco, self.stream_ptr))
+
     def _dgrad(self, L, dy, dycs, dyco, lvl, dx, dxcs, dxco, mask=None):
         """dx = conv^T(dy): the forward kernel with the transposed, flipped
         operand; mask = (y, ycs, yco): the ReLU backward of the layer below,
@@ -288,11 +297,6 @@ class UNet3D:
     def _relu_mask(self, y, ycs, yco, dy, dycs, dyco, lvl, c):
         _chk(lib.sepx_unet_relu_mask(_p(y), ycs, yco, _p(dy), dycs, dyco, self.V[lvl], c,
                                      self.stream_ptr))
-
-    def _pool(self, x, xcs, xco, lvl, c, y, ycs, yco):
-        nb = self.shape[0]
-        D, H, W = self.dims[lvl]
-        _chk(lib.sepx_unet_avgpool(_p(x), xcs, xco, nb, D, H, W, c, _p(y), ycs, yco, self.stream_ptr))
 
     def _pool_bwd(self, dy, dycs, dyco, lvl, c, dx, dxcs, dxco, acc, mask=None):
         nb = self.shape[0]
@@ -329,14 +333,11 @@ class UNet3D:
                 a["xf"].mul_(scale)
         # encoder
         self._conv(Ly["e1a"], a["x0"], 8, 0, 0, a["e1a"], 16, 0)
-        self._conv(Ly["e1b"], a["e1a"], 16, 0, 0, a["cat1"], 48, 32)
-        self._pool(a["cat1"], 48, 32, 0, 16, a["p1"], 16, 0)
+        self._conv_pool(Ly["e1b"], a["e1a"], 16, 0, 0, a["cat1"], 48, 32, a["p1"], 16, 0)
         self._conv(Ly["e2a"], a["p1"], 16, 0, 1, a["e2a"], 32, 0)
-        self._conv(Ly["e2b"], a["e2a"], 32, 0, 1, a["cat2"], 80, 48)
-        self._pool(a["cat2"], 80, 48, 1, 32, a["p2"], 32, 0)
+        self._conv_pool(Ly["e2b"], a["e2a"], 32, 0, 1, a["cat2"], 80, 48, a["p2"], 32, 0)
         self._conv(Ly["e3a"], a["p2"], 32, 0, 2, a["e3a"], 48, 0)
-        self._conv(Ly["e3b"], a["e3a"], 48, 0, 2, a["cat3"], 112, 64)
-        self._pool(a["cat3"], 112, 64, 2, 48, a["p3"], 48, 0)
+        self._conv_pool(Ly["e3b"], a["e3a"], 48, 0, 2, a["cat3"], 112, 64, a["p3"], 48, 0)
         self._conv(Ly["b4a"], a["p3"], 48, 0, 3, a["b4a"], 64, 0)
         self._conv(Ly["b4b"], a["b4a"], 64, 0, 3, a["b4b"], 64, 0)
         # decoder
