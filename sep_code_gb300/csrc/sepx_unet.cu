@@ -1563,6 +1563,18 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   CUtensorMap tm;
   if (encode_view(&tm, x, x_cstride, x_coff, cin, nb, D, H, W, kHaloX, kHaloY, 2, "conv", 16, CU_TENSOR_MAP_SWIZZLE_32B))
     return -1;
+  // packed weights: blocks of 8 x 8 (128 B), np / 8 of them per (group, tap), taps r = 3 dy + dx of a plane, dz
+  CUtensorMap tw;
+  {
+    const cuuint64_t blk = (cuuint64_t)np * 16, ngc = (cuuint64_t)cin / 8;
+    cuuint64_t dims[4] = {64, (cuuint64_t)np / 8, 9 * ngc, 3}, strides[3] = {128, blk, 9 * ngc * blk};
+    cuuint32_t box[4] = {64, (cuuint32_t)np / 8, 1, 3}, es[4] = {1, 1, 1, 1};
+    if (reinterpret_cast<uintptr_t>(wpacked) % 16) return set_error("unet conv: packed weights not 16-byte aligned");
+    const CUresult r = g_encode(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(wpacked), dims, strides, box,
+                                es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error("unet conv: cuTensorMapEncodeTiled failed (%d)", (int)r);
+  }
   ZfArgs a;
   a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.np = np; a.relu = relu;
   a.bias = bias; a.y = (__nv_bfloat16 *)y; a.y_cstride = y_cstride; a.y_coff = y_coff;
@@ -1583,19 +1595,23 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   // inside its ends two)
   const long long slots = (long long)g_num_sms * per_sm;
   const int zmax = std::min(std::min(kZfMaxZ, D), (512 / per_sm) / np);
+  auto mma_cycles = [&](int zc) {   // a tap's MMAs over a window
+    double c = 0;
+    for (int p = 0; p < zc + 2; p++) {
+      const int blk = std::min(p, zc - 1) - std::max(p - 2, 0) + 1;
+      c += std::max(32.0 + 0.25 * np * blk, 0.5 * np * blk);
+    }
+    return c;
+  };
   double best = 1e300;
   a.zc = 1;
   const int zstep = pool ? 2 : 1;   // (pooled: windows of whole plane pairs)
   for (int zc = zstep; zc <= zmax; zc += zstep) {
     const long long items = cols * ((D + zc - 1) / zc);
     const long long per = (items + slots - 1) / slots;
-    double c = 0;
-    for (int p = 0; p < zc + 2; p++) {
-      const int blk = std::min(p, zc - 1) - std::max(p - 2, 0) + 1;
-      c += std::max(32.0 + 0.25 * np * blk, 0.5 * np * blk);
-    }
-    if ((double)per * c < best) {
-      best = (double)per * c;
+    const double cost = (double)per * mma_cycles(zc);
+    if (cost < best) {
+      best = cost;
       a.zc = zc;
     }
   }
@@ -1606,6 +1622,8 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
     a.nzc = (D + a.zc - 1) / a.zc;
   }
   a.nitems = (int)(cols * a.nzc);
+  a.late_from = g_num_sms;
+  a.late = (int)(0.75 * 9 * (halo_groups(cin) / 2) * mma_cycles(a.zc));
   const auto kern = pool ? conv_zwalk_kernel<true> : conv_zwalk_kernel<false>;
   static bool attr[2] = {};
   if (!attr[pool != nullptr]) {
@@ -1617,8 +1635,7 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
     attr[pool != nullptr] = true;
   }
   const long long grid = std::min<long long>(a.nitems, slots);
-  launch_dep(kern, (unsigned)grid, kZfThreads, zf_smem_bytes(cin, np, a.nslot), st, tm,
-             (const __nv_bfloat16 *)wpacked, a);
+  launch_dep(kern, (unsigned)grid, kZfThreads, zf_smem_bytes(cin, np, a.nslot), st, tm, tw, a);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
 }
