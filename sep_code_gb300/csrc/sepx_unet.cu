@@ -1561,8 +1561,20 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   const int per_sm = std::min(fit(kZfMinSlots), 2);
   if (per_sm < 1) return 1;
   CUtensorMap tm;
-  if (encode_view(&tm, x, x_cstride, x_coff, cin, nb, D, H, W, kHaloX, kHaloY, 2, "conv", 16, CU_TENSOR_MAP_SWIZZLE_32B))
+  const bool thin = cin == 8 && x_cstride == 8 && !pool;
+  if (thin) {
+    if (reinterpret_cast<uintptr_t>(x) % 16) return set_error("unet conv: view not 16-byte aligned");
+    const cuuint64_t row = (cuuint64_t)W * 16;
+    cuuint64_t dims[4] = {(cuuint64_t)W * 8, (cuuint64_t)H, (cuuint64_t)D, (cuuint64_t)nb}, strides[3] = {row, row * H, row * H * D};
+    cuuint32_t box[4] = {8 * kHaloX, kHaloY, 1, 1}, es[4] = {1, 1, 1, 1};
+    const CUresult r = g_encode(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(x), dims, strides, box, es,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error("unet conv: cuTensorMapEncodeTiled failed (%d)", (int)r);
+  } else if (encode_view(&tm, x, x_cstride, x_coff, cin, nb, D, H, W, kHaloX, kHaloY, 2, "conv", 16,
+                         CU_TENSOR_MAP_SWIZZLE_32B)) {
     return -1;
+  }
   // packed weights: blocks of 8 x 8 (128 B), np / 8 of them per (group, tap), taps r = 3 dy + dx of a plane, dz
   CUtensorMap tw;
   {
@@ -1624,15 +1636,16 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   a.nitems = (int)(cols * a.nzc);
   a.late_from = g_num_sms;
   a.late = (int)(0.75 * 9 * (halo_groups(cin) / 2) * mma_cycles(a.zc));
-  const auto kern = pool ? conv_zwalk_kernel<true> : conv_zwalk_kernel<false>;
-  static bool attr[2] = {};
-  if (!attr[pool != nullptr]) {
+  const int form = pool ? 1 : (thin ? 2 : 0);
+  const auto kern = pool ? conv_zwalk_kernel<true, false> : (thin ? conv_zwalk_kernel<false, true> : conv_zwalk_kernel<false, false>);
+  static bool attr[3] = {};
+  if (!attr[form]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHaloMaxSmem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return set_error("unet conv: %s", cudaGetErrorString(e));
-    attr[pool != nullptr] = true;
+    attr[form] = true;
   }
   const long long grid = std::min<long long>(a.nitems, slots);
   launch_dep(kern, (unsigned)grid, kZfThreads, zf_smem_bytes(cin, np, a.nslot), st, tm, tw, a);
