@@ -824,34 +824,39 @@ struct PackJob {
   int cout, cin_p, ntap, transpose, np, kchunks;
 };
 
-__device__ __forceinline__ void pack_one(const PackJob &J, long long e) {
+// run u of 8 consecutive elements: one row n of B, eight channels of one tap
+// (channels along K are a multiple of 8).  A thread per run: its indices once,
+// its eight weights in flight (a thread per element, with 64-bit divisions,
+// took 10.7 us for the default network's 30 operands, 7.0 so).
+__device__ __forceinline__ void pack_run(const PackJob &J, uint32_t u) {
   const int nout = J.transpose ? J.cin_p : J.cout;                   // GEMM N
   const int kin = J.transpose ? ((J.cout + 7) / 8) * 8 : J.cin_p;    // channels along K
-  const int kk = (int)(e & 7);
-  const int r = (int)((e >> 3) & 7);
-  const long long rest = e >> 6;
-  const int ng = (int)(rest % (J.np / 8));
-  const long long rest2 = rest / (J.np / 8);
-  const int kg = (int)(rest2 % 8);
-  const int j = (int)(rest2 / 8);
-  const int n = ng * 8 + r;
-  const int k = j * kKC + kg * 8 + kk;
-  const int t = k / kin, c = k - t * kin;
-  float val = 0.f;
-  if (n < nout && t < J.ntap) {
-    if (!J.transpose)
-      val = J.w[((size_t)t * J.cin_p + c) * J.cout + n];
-    else if (c < J.cout)
-      val = J.w[((size_t)(J.ntap - 1 - t) * J.cin_p + n) * J.cout + c];
+  const uint32_t rest = u >> 3, kgj = rest / (uint32_t)(J.np / 8);
+  const int n = (int)(rest - kgj * (uint32_t)(J.np / 8)) * 8 + (int)(u & 7);
+  const int k = (int)kgj * 8, t = k / kin, c = k - t * kin;
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    v[i] = 0.f;
+    if (n < nout && t < J.ntap) {
+      if (!J.transpose)
+        v[i] = J.w[((size_t)t * J.cin_p + c + i) * J.cout + n];
+      else if (c + i < J.cout)
+        v[i] = J.w[((size_t)(J.ntap - 1 - t) * J.cin_p + n) * J.cout + c + i];
+    }
   }
-  J.out[e] = __float2bfloat16_rn(val);
+  __nv_bfloat16 *o = J.out + (size_t)u * 8;
+  if (reinterpret_cast<uintptr_t>(J.out) % 16 == 0) {
+    *reinterpret_cast<uint4 *>(o) = pack8(v);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; i++) o[i] = __float2bfloat16_rn(v[i]);
+  }
 }
 
 __global__ void pack_weights_kernel(const PackJob J) {
-  const long long total = (long long)J.kchunks * kKC * J.np;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x)
-    pack_one(J, e);
+  const uint32_t total = (uint32_t)((long long)J.kchunks * kKC * J.np / 8);
+  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) pack_run(J, u);
 }
 
 // up to kMaxPackJobs packings in one launch: blockIdx.y picks the job
@@ -861,10 +866,8 @@ struct PackJobs {
 };
 __global__ void pack_weights_many_kernel(const __grid_constant__ PackJobs P) {
   const PackJob &J = P.j[blockIdx.y];
-  const long long total = (long long)J.kchunks * kKC * J.np;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x)
-    pack_one(J, e);
+  const uint32_t total = (uint32_t)((long long)J.kchunks * kKC * J.np / 8);
+  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) pack_run(J, u);
 }
 
 // ---------------------------------------------------------------------------
@@ -1964,7 +1967,7 @@ int sepx_unet_pack_weights(const float *w, int cout, int cin_p, int ntap, int tr
     return set_error("unet pack: channels (%d -> %d) unsupported", kin, nout);
   const int np = np_of(nout), kch = (ntap * kin + kKC - 1) / kKC;
   PackJob J{w, (__nv_bfloat16 *)out, cout, cin_p, ntap, transpose, np, kch};
-  pack_weights_kernel<<<grid_for((long long)kch * kKC * np), 256, 0, (cudaStream_t)stream>>>(J);
+  pack_weights_kernel<<<grid_for((long long)kch * kKC * np / 8), 256, 0, (cudaStream_t)stream>>>(J);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet pack: %s", cudaGetErrorString(e));
 }
@@ -1986,7 +1989,7 @@ int sepx_unet_pack_weights_many(int njobs, const float *const *w, void *const *o
     P.j[i] = PackJob{w[i], (__nv_bfloat16 *)out[i], cout[i], cin_p[i], ntap[i], tr, np, kch};
     most = std::max(most, (long long)kch * kKC * np);
   }
-  const long long bx = std::min<long long>((most + 255) / 256, 64);
+  const long long bx = std::min<long long>((most / 8 + 255) / 256, 64);
   pack_weights_many_kernel<<<dim3((unsigned)bx, (unsigned)njobs), 256, 0, (cudaStream_t)stream>>>(P);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet pack: %s", cudaGetErrorString(e));
