@@ -1659,11 +1659,16 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
 // The convolution with streamed weights (sepx_unet_kstream.inc): 3x3x3 layers
 // whose weights do not fit in shared memory or whose planes are smaller than a
 // tile, where channels come in pairs of groups (a K16 step stays in one tap),
-// the planes a K range reads fit in shared memory, and staging them moves at
-// most half of what the gather kernel copies for the range and the tile's real
-// voxels.  Measured (gather -> this, kernel, us): 112 -> 48 on 32^3 voxels 91
-// -> 29, 48 -> 112 on 4 x 16^3 32 -> 19, both beyond the line; short of it (K
-// ranges of 3 chunks) 64 -> 64 on 16^3 10.5 -> 11.2, on 4 x 8^3 8.1 -> 8.8.
+// the planes a K range reads fit in shared memory, staging them moves at most
+// 0.4 of what the gather kernel copies for the range and the tile's real
+// voxels, and a range's MMAs take at least 1400 cycles (an item's fixed costs).
+// Measured (gather -> this, us a call; share staged, cycles): 112 -> 48 on 32^3
+// voxels 91 -> 30 (0.20, 4224), 64 -> 64 on 40 x 12 x 40 26.4 -> 17.5 (0.26,
+// 2592), 32 -> 48 on 116 x 12 x 122 83 -> 61 (0.22, 2376), 48 -> 16 on 68 x 12 x
+// 40 27.9 -> 22.5 (0.26, 1584); at the lines 112 -> 48 on 2 x 30 x 9 x 51 53.5 ->
+// 53.3 (0.36), 48 -> 64 on 30 x 9 x 40 18.4 -> 18.4 (1152); short of them 16 ->
+// 16 on 2 x 14 x 9 x 100 11.6 -> 20.9 (0.33, 576), 16 -> 32 on 50 x 9 x 100 15.9
+// -> 26.6 (1080), 64 -> 64 on 16^3, the kernels, 10.5 -> 11.2 (0.47).
 // Returns 1 where it does not apply.
 int conv_kstream(View x, int nb, int D, int H, int W, int cin, const void *wpacked, const float *bias, int cout,
                  int np, int relu, void *y, int y_cstride, int y_coff, float *yf, const float *resid, View mask,
@@ -1682,7 +1687,8 @@ int conv_kstream(View x, int nb, int D, int H, int W, int cin, const void *wpack
     span = std::max(span, (k1 - 1) / per9 - k0 / per9 + 1);
   }
   const double staged = (double)cols * D * span * (kHaloX * kHaloY) * cin, gathered = (double)nb * D * H * W * kper * kKC;
-  if (2 * staged > gathered) return 1;
+  const int steps = std::min(kper * (kKC / 16), 3 * per9);
+  if (2.5 * staged > gathered || steps * std::max(32.0 + 0.25 * np, 0.5 * np) < 1400) return 1;
   if (unet_dev_init()) return -1;
   auto fit = [&](int nring, int nw) {
     const size_t sm = ks_smem_bytes(cin, np, nring, nw);

@@ -22,9 +22,9 @@ torch = pytest.importorskip("torch")
 # planes, ragged rows and columns, planes smaller than a tile (H = 8, W = 4);
 # the widest columns (np = 128) and plane slots (160, 208 channels); two layers
 # short of the line (the gather kernel takes them)
-CASES = [(112, 48, 2, 12, 32, 16), (112, 48, 2, 13, 31, 16), (48, 112, 2, 12, 32, 16), (128, 128, 1, 24, 32, 16),
-         (208, 16, 1, 24, 32, 16), (112, 48, 1, 41, 33, 40), (48, 112, 2, 23, 31, 40), (160, 16, 1, 19, 48, 56),
-         (16, 128, 2, 60, 8, 48), (32, 1, 1, 700, 16, 4), (112, 48, 1, 1, 16, 8), (64, 64, 2, 8, 8, 16)]
+CASES = [(112, 48, 2, 12, 32, 24), (112, 48, 2, 13, 31, 24), (48, 112, 2, 12, 32, 16), (128, 128, 1, 24, 32, 24),
+         (208, 16, 1, 24, 32, 24), (112, 48, 1, 41, 33, 40), (48, 112, 2, 23, 31, 40), (160, 16, 1, 19, 48, 56),
+         (16, 128, 2, 60, 8, 48), (32, 1, 1, 700, 16, 4), (112, 48, 1, 1, 16, 8), (16, 16, 2, 22, 9, 31)]
 
 
 @pytest.mark.parametrize("cin,cout,nb,D,H,W", CASES)
