@@ -108,6 +108,10 @@ int sepx_unet_bias_grad(const void *dy, int dy_cstride, int dy_coff, long long V
 /* FP32 single-channel volume * scale -> channel coff of a BF16 view (8-channel group, rest 0) */
 int sepx_unet_to_bf16(const float *in, long long V, float scale, void *y, int y_cstride, int y_coff,
                       void *stream);
+/* The same, and xf[v] = in[v] * scale (FP32, NULL: not written): the network's
+ * input and its residual in one pass */
+int sepx_unet_input(const float *in, long long V, float scale, void *y, int y_cstride, int y_coff, float *xf,
+                    void *stream);
 /* *loss += mean (out - target)^2 (FP64); g (BF16, channel 0 of 8) = d loss / d out */
 int sepx_unet_mse(const float *out, const float *target, long long V, void *g, int g_cstride,
                   double *loss, void *stream);

@@ -54,6 +54,7 @@ _SIGS = {
     "sepx_unet_relu_mask": [_vp, _i, _i, _vp, _i, _i, _ll, _i, _vp],
     "sepx_unet_bias_grad": [_vp, _i, _i, _ll, _i, _vp, _vp],
     "sepx_unet_to_bf16": [_vp, _ll, _f, _vp, _i, _i, _vp],
+    "sepx_unet_input": [_vp, _ll, _f, _vp, _i, _i, _vp, _vp],
     "sepx_unet_mse": [_vp, _vp, _ll, _vp, _i, _vp, _vp],
     "sepx_unet_adam": [_vp, _vp, _vp, _vp, _ll, _f, _f, _f, _f, _i, _vp],
     "sepx_unet_adam_dev": [_vp, _vp, _vp, _vp, _ll, _vp, _vp],
@@ -326,11 +327,7 @@ class UNet3D:
         self._alloc(nb, D, H, W)
         a, Ly = self.a, {L.name: L for L in LAYERS}
         V0 = self.V[0]
-        _chk(lib.sepx_unet_to_bf16(_p(xf), V0, scale, _p(a["x0"]), 8, 0, self.stream_ptr))
-        with self.torch.cuda.stream(self.stream):
-            a["xf"].copy_(xf.reshape(-1))
-            if scale != 1.0:
-                a["xf"].mul_(scale)
+        _chk(lib.sepx_unet_input(_p(xf), V0, scale, _p(a["x0"]), 8, 0, _p(a["xf"]), self.stream_ptr))
         # encoder
         self._conv(Ly["e1a"], a["x0"], 8, 0, 0, a["e1a"], 16, 0)
         self._conv_pool(Ly["e1b"], a["e1a"], 16, 0, 0, a["cat1"], 48, 32, a["p1"], 16, 0)
