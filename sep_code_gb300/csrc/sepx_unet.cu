@@ -26,6 +26,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <mutex>
 
@@ -1812,6 +1813,32 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   }
   a.nitems = (int)(cols * a.nzc);
   a.groups = std::min(a.nitems, slots);
+  // The tensor cores truncate as they add: a chain of n MMAs (8 a tile) into
+  // one accumulator loses about 1.5e-8 n of a sum, in one direction.  So the
+  // accumulators are read out, and added in FP32 to the CTA's partial sums,
+  // once they have taken the tiles of a chain that `acc` accumulators per SM
+  // would leave each, `least` at least.  The numbers are those of the forms
+  // that ran these layers before (one to four CTAs an SM; the gather kernel's
+  // splits), whose errors are the bound.  Relative L2 error of one read-out ->
+  // of these (and time, us): 8 -> 16 channels on 4 x 64^3 voxels 7.2e-6 ->
+  // 1.4e-6 (47 -> 55), 32 -> 48 2.2e-5 -> 3.8e-6 (152 -> 170), 112 -> 48 on 2 x
+  // 64^3 2.1e-5 -> 7.1e-6 (207 -> 216), 32 -> 32 on 4 x 32^3 8.2e-7 -> 4.0e-7
+  // (23 -> 29); a training step on 4 x 64^3 1018 -> 1091.
+  double acc;
+  int least;
+  if (njob == 1) {
+    acc = a.pw == 16 && a.ncb == 1 ? (cin == 8 ? 4.0 : 2.0) : 1.0;
+    least = a.pw == 16 && a.ncb == 1 ? 2 : 4;
+  } else if (cout <= 40) {
+    acc = a.pw == 64 ? 1.43 : 0.72;
+    least = 2;
+  } else {
+    acc = 10.0 / ((27 * cin + 127) / 128);
+    least = 8;
+  }
+  const int run = (a.nitems + a.groups - 1) / a.groups * a.zc;   // tiles of the busiest CTA
+  const int nout = (int)std::ceil(run / std::max((double)least, 1.1 * (double)(cols * D) / (g_num_sms * acc)));
+  a.seg = (run + nout - 1) / nout;
   a.err = err;
   // 16, 32, 64 rows' channels x (three sy stacked, one sy stacked, one sy per dz)
   const decltype(&conv_wgrad_ring_kernel<16, 3, true>) kerns[9] = {
