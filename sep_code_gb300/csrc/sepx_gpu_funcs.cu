@@ -1096,10 +1096,7 @@ int sepx_dot_f32(const float *a, const float *b, long long n, double *result) {
   RET(need_span(a, n, "sepx_dot_f32 a"));   // b == NULL: the sum of a
   RET(need_device());
   // the result goes straight to mapped host memory: no copy behind the kernel
-  if (!G.d_dot) {
-    CK(cudaMalloc((void **)&G.d_dot, vec_dot_scratch_doubles() * sizeof(double)));
-    CK(cudaMemsetAsync(G.d_dot, 0, vec_dot_scratch_doubles() * sizeof(double), G.stream));
-  }
+  if (!G.d_dot) CK(alloc_zeroed(&G.d_dot, vec_dot_scratch_doubles(), G.stream));
   if (!G.h_dot) CK(cudaHostAlloc((void **)&G.h_dot, sizeof(double), cudaHostAllocMapped));
   CKL(vec_dot(a, b, n, G.d_dot, G.h_dot, G.stream));
   CK(cudaStreamSynchronize(G.stream));
