@@ -49,12 +49,12 @@ int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, 
                               const void *mask, int mask_cstride, int mask_coff, void *stream);
 /* 3x3x3 layers whose planes are at least 16 x 8 voxels and whose packed
  * weights and input halo fit in 227 KB of shared memory run on the z-walk
- * kernel (at most 80 output channels) or the halo-staged kernel (the same
- * bits), others with streamed weights where that moves less than the gather
- * kernel (the same bits), and the weight gradients of 3x3x3 layers with at
- * most 64 output and 112 input channels on the tap-stacked kernels;
- * enable = 0 sends every layer to the per-tap gather kernels.  Returns the
- * previous setting. */
+ * kernel (at most 80 output channels, but not 40 -> 65 to 80) or the
+ * halo-staged kernel (the same bits), others with streamed weights where that
+ * moves less than the gather kernel (the same bits), and the weight gradients
+ * of 3x3x3 layers with at most 64 output and 112 input channels on the ring
+ * tap-stacked kernel; enable = 0 sends every layer to the per-tap gather
+ * kernels.  Returns the previous setting. */
 int sepx_unet_set_halo(int enable);
 /* Weight-gradient kernel choice (with the halo-staged kernels enabled):
  * 2 (default) the ring tap-stacked kernel (cin <= 112, cout <= 64), else

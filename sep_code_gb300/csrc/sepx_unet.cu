@@ -1549,9 +1549,11 @@ struct PoolOut {
 };
 
 // The z-walk convolution (sepx_unet_zwfwd.inc): every layer the halo-staged
-// kernel takes whose three column blocks fit one MMA (3 x np <= 256; it
-// measured 3.3 to 5.3 times as fast on those).  Returns 1 where it does not
-// apply (np >= 96: the halo-staged kernel).
+// kernel takes whose three column blocks fit one MMA (3 x np <= 256) and whose
+// weights leave room for a ring of four slots (it measured 3.3 to 5.3 times as
+// fast on those).  Returns 1 where it does not apply: np 96 to 128 with cin up
+// to 24, np 96 or 112 with cin 32, and np 80 with cin 40 (226 KB of weights and
+// halo fit, 249 KB of weights and ring do not) stay on the halo-staged kernel.
 int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
                const void *wpacked, const float *bias, int cout, int np, int relu, void *y, int y_cstride,
                int y_coff, float *yf, const float *resid, View mask, int *err, const PoolOut *pool, cudaStream_t st) {
