@@ -150,8 +150,7 @@ __global__ void __launch_bounds__(kDotThreads)
   }
 }
 
-// ---- elementwise operations on N elements at a time, y = op(y, x1, x2): 8 or 4
-// where every pointer is 16-byte aligned, else (and past the last four) 1 ----
+// ---- elementwise operations on N elements at a time, y = op(y, x1, x2) ----
 struct OpFill {
   float v;
   template <int N>
@@ -214,49 +213,57 @@ struct OpMult {
   }
 };
 
-template <bool Y, bool X1, bool X2, class OP>
-__global__ void __launch_bounds__(256) map_kernel(float *y, const float *x1, const float *x2, long long n, int vec,
-                                                  OP op) {
+// A thread takes U * W elements a step, W neighbours per access (4: every
+// pointer 16-byte aligned), U accesses a grid's width apart; then W at a time,
+// then, past the last four, one.
+template <int W, int U, bool Y, bool X1, bool X2, class OP>
+__global__ void __launch_bounds__(256) map_kernel(float *y, const float *x1, const float *x2, long long n, OP op) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-  long long i0 = t;
-  if (vec) {
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const long long n4 = n >> 2;
-    // eight elements a step where there are as many: shorter slow paths of the
-    // conversions are predicated instead of branched around
-    long long i = t;
-    for (; i + stride < n4; i += 2 * stride) {
-      float v[8], p[8], q[8];
+  const long long nu = n / W;
+  auto load = [](const float *p, long long k, float *v) {
+    if constexpr (W == 4) {
+      const float4 q = reinterpret_cast<const float4 *>(p)[k];
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+      v[0] = p[k];
+    }
+  };
+  auto store = [](float *p, long long k, const float *v) {
+    if constexpr (W == 4)
+      reinterpret_cast<float4 *>(p)[k] = make_float4(v[0], v[1], v[2], v[3]);
+    else
+      p[k] = v[0];
+  };
+  long long i = t;
+  if constexpr (U > 1) {
+    for (; i + (U - 1) * stride < nu; i += U * stride) {
+      float v[U * W] = {}, p[U * W] = {}, q[U * W] = {};
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const long long k = i + h * stride;
-        const float4 a = Y ? reinterpret_cast<const float4 *>(y)[k] : z;
-        const float4 b = X1 ? reinterpret_cast<const float4 *>(x1)[k] : z;
-        const float4 c = X2 ? reinterpret_cast<const float4 *>(x2)[k] : z;
-        v[4 * h] = a.x; v[4 * h + 1] = a.y; v[4 * h + 2] = a.z; v[4 * h + 3] = a.w;
-        p[4 * h] = b.x; p[4 * h + 1] = b.y; p[4 * h + 2] = b.z; p[4 * h + 3] = b.w;
-        q[4 * h] = c.x; q[4 * h + 1] = c.y; q[4 * h + 2] = c.z; q[4 * h + 3] = c.w;
+      for (int h = 0; h < U; h++) {
+        if (Y) load(y, i + h * stride, v + W * h);
+        if (X1) load(x1, i + h * stride, p + W * h);
+        if (X2) load(x2, i + h * stride, q + W * h);
       }
       op(v, p, q);
-      reinterpret_cast<float4 *>(y)[i] = make_float4(v[0], v[1], v[2], v[3]);
-      reinterpret_cast<float4 *>(y)[i + stride] = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+      for (int h = 0; h < U; h++) store(y, i + h * stride, v + W * h);
     }
-    if (i < n4) {
-      const float4 a = Y ? reinterpret_cast<const float4 *>(y)[i] : z;
-      const float4 b = X1 ? reinterpret_cast<const float4 *>(x1)[i] : z;
-      const float4 c = X2 ? reinterpret_cast<const float4 *>(x2)[i] : z;
-      float v[4] = {a.x, a.y, a.z, a.w};
-      const float p[4] = {b.x, b.y, b.z, b.w}, q[4] = {c.x, c.y, c.z, c.w};
-      op(v, p, q);
-      reinterpret_cast<float4 *>(y)[i] = make_float4(v[0], v[1], v[2], v[3]);
-    }
-    i0 = (n4 << 2) + t;
   }
-  for (long long i = i0; i < n; i += stride) {
-    float v[1] = {Y ? y[i] : 0.f};
-    const float p[1] = {X1 ? x1[i] : 0.f}, q[1] = {X2 ? x2[i] : 0.f};
+  for (; i < nu; i += stride) {
+    float v[W] = {}, p[W] = {}, q[W] = {};
+    if (Y) load(y, i, v);
+    if (X1) load(x1, i, p);
+    if (X2) load(x2, i, q);
     op(v, p, q);
-    y[i] = v[0];
+    store(y, i, v);
+  }
+  if constexpr (W > 1) {
+    for (long long k = nu * W + t; k < n; k += stride) {
+      float v[1] = {Y ? y[k] : 0.f};
+      const float p[1] = {X1 ? x1[k] : 0.f}, q[1] = {X2 ? x2[k] : 0.f};
+      op(v, p, q);
+      y[k] = v[0];
+    }
   }
 }
 
@@ -279,10 +286,26 @@ static int grid_for(long long n) {
   return (int)(g < 2048 ? (g < 1 ? 1 : g) : 2048);
 }
 
+// Eight elements a thread and step keep the conversions' slow path a real
+// branch and the loads of a step in flight, 16 bytes at a time where the
+// pointers allow; shorter vectors take one element a thread, as eight would
+// leave most SMs, and their FP64 pipes, idle.  Measured (one -> eight, us; y =
+// a x1 + b x2): 5000 elements 3.3 -> 6.1, 180 000 4.1 -> 6.1, 262 144 6.1 ->
+// 5.1, 3 M 26.7 -> 16.4, 60 M 472 -> 252; not 16-byte aligned 400 000 6.1 ->
+// 8.2, 600 000 8.2 -> 8.2, 3 M 26.7 -> 18.5, 60 M 471 -> 252.  (Unaligned
+// vectors in the eights' kernel one element at a time: y += x of 60 M 336 us,
+// half the warps of a kernel of its own, 166; 128 so.)
 template <bool Y, bool X1, bool X2, class OP>
 static cudaError_t map(float *y, const float *x1, const float *x2, long long n, OP op, cudaStream_t st) {
-  const int vec = al16(y) && (!X1 || al16(x1)) && (!X2 || al16(x2));
-  map_kernel<Y, X1, X2><<<grid_for(vec ? (n + 7) / 8 : n), 256, 0, st>>>(y, x1, x2, n, vec, op);
+  const bool al = al16(y) && (!X1 || al16(x1)) && (!X2 || al16(x2));
+  const bool eights = n >= (al ? 1LL << 18 : 1LL << 19);
+  const int grid = grid_for(eights ? (n + 7) / 8 : n);
+  if (!eights)
+    map_kernel<1, 1, Y, X1, X2><<<grid, 256, 0, st>>>(y, x1, x2, n, op);
+  else if (al)
+    map_kernel<4, 2, Y, X1, X2><<<grid, 256, 0, st>>>(y, x1, x2, n, op);
+  else
+    map_kernel<1, 8, Y, X1, X2><<<grid, 256, 0, st>>>(y, x1, x2, n, op);
   return cudaGetLastError();
 }
 
