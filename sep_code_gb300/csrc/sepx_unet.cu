@@ -29,6 +29,7 @@
 #include <cmath>
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 
 #include "sepx_common.h"
 #include "sepx_device.cuh"
@@ -895,16 +896,18 @@ __global__ void __launch_bounds__(256, 3) conv1x1_kernel(View x, long long V, co
   }
   for (int i = threadIdx.x; i < COUT; i += blockDim.x) bs[i] = bias ? bias[i] : 0.f;
   __syncthreads();
-  // NV voxels per thread and pass: the weights, read again from shared memory
-  // (in registers they cost a memory-bound kernel its warps), bound the kernel
-  // with one (16 outputs, 4 x 64^3 voxels: 28.6 us, 23.9 with two)
-  constexpr int NV = COUT > 1 ? 2 : 1;
+  // two voxels per thread and pass where there are as many: the weights, read
+  // again from shared memory (in registers they cost a memory-bound kernel its
+  // warps), bound the kernel with one (16 outputs, 4 x 64^3 voxels: 28.6 us,
+  // 23.9 with two; 2 x 256^2 voxels, where no thread has a second: 6.2 us, 7.2
+  // with the first one twice)
   const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long v0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; v0 < V; v0 += NV * step) {
+  auto pass = [&](long long v0, auto nvc) {
+    constexpr int NV = decltype(nvc)::value;
     float xin[NV][CIN];
 #pragma unroll
     for (int j = 0; j < NV; j++) {
-      const long long v = v0 + j * step < V ? v0 + j * step : v0;
+      const long long v = v0 + j * step;
 #pragma unroll
       for (int g = 0; g < CIN / 8; g++) {
         const uint4 q = *reinterpret_cast<const uint4 *>(x.p + v * x.cstride + x.coff + 8 * g);
@@ -942,7 +945,6 @@ __global__ void __launch_bounds__(256, 3) conv1x1_kernel(View x, long long V, co
 #pragma unroll
       for (int j = 0; j < NV; j++) {
         const long long v = v0 + j * step;
-        if (v >= V) break;
         if constexpr (NG == 8) {
           if (mask.p) mask8(mask.p + v * mask.cstride + mask.coff + n0, acc[j]);
           if (y) *reinterpret_cast<uint4 *>(y + v * y_cstride + y_coff + n0) = pack8(acc[j]);
@@ -953,7 +955,11 @@ __global__ void __launch_bounds__(256, 3) conv1x1_kernel(View x, long long V, co
         }
       }
     }
-  }
+  };
+  constexpr int NV = COUT > 1 ? 2 : 1;
+  long long v0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  for (; v0 + (NV - 1) * step < V; v0 += NV * step) pass(v0, std::integral_constant<int, NV>());
+  if (NV > 1 && v0 < V) pass(v0, std::integral_constant<int, 1>());
 }
 
 // part[block][(c, n)] = sum over the block's voxels of x[v][c] dy[v][n], and

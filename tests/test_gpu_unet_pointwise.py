@@ -1,0 +1,58 @@
+"""The U-Net's pointwise kernels where their forms change: nearest upsampling of
+packed 8-channel volumes (two children per 32-byte store, if the volume is
+aligned for it), the 8 -> 16 channel 1x1x1 convolution around the number of
+threads of its grid (two voxels a thread, or one), and the network's input with
+and without the FP32 copy.
+
+Upsampling and the input are copies: the bits of PyTorch's on the CPU.  The
+convolution adds 8 products and a bias in FP32, nine roundings of at most 2^-24
+of the terms' sum: 9 * 2^-24 = 5.4e-7 of it; and a voxel's result does not
+depend on the volume around it: the same bits in pieces."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+GRID = 4 * 152 * 256   # threads of the 1x1x1 convolution's largest grid
+
+
+def _net():
+    from sep_code_gb300 import unet as net
+    from sep_code_gb300._lib import lib
+    lib.sepx_setup_cuda(1)
+    return net, lib, lib.sepx_get_stream()
+
+
+@pytest.mark.parametrize("V", [1, 255, GRID - 1, GRID, GRID + 1, 2 * GRID, 2 * GRID + 5])
+def test_conv_8_16_around_the_grid(V):
+    net, lib, st = _net()
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x = torch.randn((V, 8), device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn((1, 8, 16), device="cuda", generator=g)
+    b = torch.randn(16, device="cuda", generator=g)
+    m = torch.randn((V, 16), device="cuda", generator=g).to(torch.bfloat16)
+    pk = torch.zeros(lib.sepx_unet_packed_elems(16, 8, 1, 0), dtype=torch.bfloat16, device="cuda")
+    y, yp = (torch.full((V, 24), -3.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    yf = torch.zeros((V, 16), device="cuda")
+    torch.cuda.synchronize()
+    net._chk(lib.sepx_unet_pack_weights(net._p(w), 16, 8, 1, 0, net._p(pk), st))
+
+    def conv(v0, v1, out, relu, mask, f32):
+        net._chk(lib.sepx_unet_conv_fwd_masked(net._p(x[v0:]), 8, 0, 1, 1, 1, v1 - v0, 8, 1, net._p(pk), net._p(b), 16,
+                                               relu, net._p(out[v0:]), 24, 8, f32, None,
+                                               net._p(mask[v0:]) if mask is not None else None, 16 if mask is not None else 0,
+                                               0, st))
+    conv(0, V, y, 0, None, net._p(yf))
+    lib.sepx_synchronize()
+    xs, ws = x.double(), w[0].to(torch.bfloat16).double()
+    want, mag = xs @ ws + b.double(), xs.abs() @ ws.abs() + b.double().abs()
+    assert bool(((yf.double() - want).abs() <= 9 * 2.0 ** -24 * mag).all())
+    assert torch.equal(y[:, 8:], yf.to(torch.bfloat16)) and bool((y[:, :8] == -3.0).all())
+    conv(0, V, y, 1, m, None)
+    step = 100000
+    for v0 in range(0, V, step):
+        conv(v0, min(v0 + step, V), yp, 1, m, None)
+    lib.sepx_synchronize()
+    assert torch.equal(y.view(torch.int16), yp.view(torch.int16))
