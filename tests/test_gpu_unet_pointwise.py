@@ -25,6 +25,23 @@ def _net():
     return net, lib, lib.sepx_get_stream()
 
 
+@pytest.mark.parametrize("off", [0, 8, 16])
+@pytest.mark.parametrize("nb,D,H,W", [(1, 1, 1, 1), (2, 3, 5, 7), (1, 8, 33, 64)])
+def test_upsample_packed_bits(nb, D, H, W, off):
+    net, lib, st = _net()
+    x = torch.randn((nb, D, H, W, 8), generator=torch.Generator().manual_seed(W + off)).to(torch.bfloat16)
+    n = x.numel() * 8
+    y = torch.full((n + 32,), 5.0, dtype=torch.bfloat16, device="cuda")
+    xd, yd = x.cuda(), y[off:]
+    torch.cuda.synchronize()
+    net._chk(lib.sepx_unet_upsample(net._p(xd), 8, 0, nb, D, H, W, 8, net._p(yd), 8, 0, st))
+    lib.sepx_synchronize()
+    want = x.repeat_interleave(2, 1).repeat_interleave(2, 2).repeat_interleave(2, 3).reshape(-1)
+    got = y.cpu()
+    assert torch.equal(got[off:off + n].view(torch.int16), want.view(torch.int16))
+    assert (got[:off] == 5.0).all() and (got[off + n:] == 5.0).all()
+
+
 @pytest.mark.parametrize("V", [1, 255, GRID - 1, GRID, GRID + 1, 2 * GRID, 2 * GRID + 5])
 def test_conv_8_16_around_the_grid(V):
     net, lib, st = _net()
