@@ -1274,6 +1274,7 @@ __global__ void bias_sum_kernel(const float *__restrict__ part, int blocks, int 
 // FP32 volume (one channel) -> BF16 channel-last view channel 0, other
 // channels of the 8-channel group zero; scale applied; xf (or NULL): the scaled
 // volume in FP32 too
+template <bool XF>
 __global__ void to_bf16_kernel(const float *in, long long V, float scale, __nv_bfloat16 *y,
                                int y_cstride, int y_coff, float *xf) {
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V;
@@ -1281,7 +1282,7 @@ __global__ void to_bf16_kernel(const float *in, long long V, float scale, __nv_b
     __align__(16) __nv_bfloat16 o[8];
     const float x = in[v] * scale;
     o[0] = __float2bfloat16_rn(x);
-    if (xf) xf[v] = x;
+    if (XF) xf[v] = x;
 #pragma unroll
     for (int i = 1; i < 8; i++) o[i] = __float2bfloat16_rn(0.f);
     *reinterpret_cast<uint4 *>(y + v * y_cstride + y_coff) = *reinterpret_cast<const uint4 *>(o);
@@ -2365,8 +2366,8 @@ int sepx_unet_input(const float *in, long long V, float scale, void *y, int y_cs
   if (V < 0) return set_error("unet to_bf16: negative length");
   if (V == 0) return 0;
   if (need_dev(in, "to_bf16 in") || need_dev(y, "to_bf16 y")) return -1;
-  to_bf16_kernel<<<grid_for(V), 256, 0, (cudaStream_t)stream>>>(in, V, scale, (__nv_bfloat16 *)y,
-                                                                y_cstride, y_coff, xf);
+  (xf ? to_bf16_kernel<true> : to_bf16_kernel<false>)<<<grid_for(V), 256, 0, (cudaStream_t)stream>>>(
+      in, V, scale, (__nv_bfloat16 *)y, y_cstride, y_coff, xf);
   return cudaGetLastError() == cudaSuccess ? 0 : set_error("unet to_bf16: launch failed");
 }
 

@@ -73,3 +73,21 @@ def test_conv_8_16_around_the_grid(V):
         conv(v0, min(v0 + step, V), yp, 1, m, None)
     lib.sepx_synchronize()
     assert torch.equal(y.view(torch.int16), yp.view(torch.int16))
+
+
+@pytest.mark.parametrize("V", [1, 777, 300001])
+def test_input_with_and_without_the_float_copy(V):
+    net, lib, st = _net()
+    x = torch.randn(V, generator=torch.Generator().manual_seed(V))
+    xd = x.cuda()
+    y = [torch.full((V, 16), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    xf = torch.zeros(V, device="cuda")
+    torch.cuda.synchronize()
+    net._chk(lib.sepx_unet_to_bf16(net._p(xd), V, 0.3, net._p(y[0]), 16, 8, st))
+    net._chk(lib.sepx_unet_input(net._p(xd), V, 0.3, net._p(y[1]), 16, 8, net._p(xf), st))
+    lib.sepx_synchronize()
+    s = x * np.float32(0.3)
+    assert torch.equal(xf.cpu(), s)
+    for t in y:
+        t = t.cpu()
+        assert torch.equal(t[:, 8], s.to(torch.bfloat16)) and (t[:, :8] == 7.0).all() and (t[:, 9:] == 0).all()
