@@ -35,13 +35,11 @@
 #include "sepx_device.cuh"
 #include "sepx_tc.cuh"
 #include "sepx_unet.h"
+#include "sepx_unet_plan.h"
 
 namespace sepx {
 
-constexpr int kTM = 128;   // GEMM rows per CTA (tensor-memory lanes)
-constexpr int kKC = 64;    // K per pipeline stage (8 K groups of 8)
 constexpr int kUThreads = 128;
-constexpr int kMaxN = 128;
 
 struct View {
   const __nv_bfloat16 *p;
@@ -354,10 +352,6 @@ __global__ void conv_finish_kernel(const float *kpart, int splits, long long V, 
 // memory; the CTA walks tiles (persistent), prefetching the next tile's halo
 // into the other of two buffers while the current one is computed.
 // ---------------------------------------------------------------------------
-constexpr int kHaloX = 10, kHaloY = 18, kHaloZ = 3;
-constexpr int kHaloGS = 8704;   // bytes per channel group (8640 rounded up to 128)
-constexpr int kTileY = 16, kTileX = 8;
-
 struct HaloArgs {
   int nb, D, H, W, cin, cout, np, relu;
   const float *bias;
@@ -373,14 +367,6 @@ struct HaloArgs {
   View mask;           // ReLU-backward mask (mask.p NULL: none)
 };
 
-// channel groups held per halo buffer: cin/8 rounded up to even (an odd
-// count gets one all-zero group, the channel box lying wholly outside x)
-__host__ __device__ constexpr int halo_groups(int cin) { return ((cin / 8) + 1) & ~1; }
-
-__host__ __device__ constexpr size_t halo_smem_bytes(int cin, uint32_t wbytes, int nbuf) {
-  return (size_t)wbytes + (size_t)nbuf * (size_t)halo_groups(cin) * kHaloGS + 256 + 128;
-}
-
 // Warp roles: warp 4 (lane 0) loads the weights and the halos and issues the
 // MMAs; warps 0-3 run the epilogue (warp w owns tensor-memory lanes
 // 32w..32w+31 = tile rows).  Two accumulators in tensor memory: the MMAs of
@@ -389,7 +375,6 @@ __host__ __device__ constexpr size_t halo_smem_bytes(int cin, uint32_t wbytes, i
 // halo buffer b are done (tcgen05.commit), acc[a] accumulator a complete
 // (commit), afree[a] accumulator a read by the 4 epilogue warps, wbar weights.
 constexpr int kHaloThreads = 160;
-constexpr int kMaxPairs = 8;   // channel-group pairs of one halo (up to 128 channels)
 
 __global__ void __launch_bounds__(kHaloThreads) conv_halo_kernel(const __grid_constant__ CUtensorMap tmx,
                                                                  const __nv_bfloat16 *wp,
@@ -1415,15 +1400,10 @@ int check_conv_args(int cin, int cstride, int coff, int cout, int ntap) {
 }
 int np_of(int cout) { return ((cout + 15) / 16) * 16; }
 
-// The halo-staged convolution takes 3x3x3 layers whose planes hold at least
-// one 16 x 8 tile and whose weights and a halo buffer fit in the 227 KB of
-// shared memory a CTA may have (one CTA per SM for the largest of them).
-constexpr size_t kHaloMaxSmem = 227 * 1024;
 bool g_halo_enabled = true;
 int g_wgrad_form = 2;   // 2: ring, else per-tile TMA, else gather; 1: per-tile TMA, else gather; 0: gather
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
-int g_num_sms = 0;
-size_t g_smem_per_sm = 0, g_smem_reserved = 0;
+UnetDev g_dev;
 
 // the tensor-map encoder and the device figures the persistent grids are sized from
 int unet_dev_init() {
@@ -1436,12 +1416,12 @@ int unet_dev_init() {
     return set_error("unet conv: cuTensorMapEncodeTiled is unavailable");
   int dev = 0, smem_sm = 0, resv = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&g_dev.num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&resv, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess)
     return set_error("unet conv: cannot query the device");
-  g_smem_per_sm = (size_t)smem_sm;
-  g_smem_reserved = (size_t)resv;
+  g_dev.smem_per_sm = (size_t)smem_sm;
+  g_dev.smem_reserved = (size_t)resv;
   g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
   return 0;
 }
@@ -1526,8 +1506,8 @@ int conv_halo(const void *x, int x_cstride, int x_coff, int nb, int D, int H, in
   // persistent grid must all be resident): two halo buffers unless one
   // buffer fits two CTAs per SM where two buffers fit only one
   auto fit = [&](int nbuf) {
-    const size_t per = ((halo_smem_bytes(cin, wbytes, nbuf) + 127) / 128) * 128 + g_smem_reserved;
-    return (int)(g_smem_per_sm / per);
+    const size_t per = ((halo_smem_bytes(cin, wbytes, nbuf) + 127) / 128) * 128 + g_dev.smem_reserved;
+    return (int)(g_dev.smem_per_sm / per);
   };
   // two or more channel-group pairs: one buffer pipelined pair by pair;
   // a single pair: two buffers where they still leave two CTAs per SM
@@ -1553,7 +1533,7 @@ int conv_halo(const void *x, int x_cstride, int x_coff, int nb, int D, int H, in
   // tensor memory: two accumulators per CTA, at most 512 columns per SM
   const int ncols = 2 * (np <= 32 ? 32 : (np <= 64 ? 64 : 128));
   if (per_sm * ncols > 512) per_sm = 512 / ncols;
-  long long grid = (long long)g_num_sms * per_sm;
+  long long grid = (long long)g_dev.num_sms * per_sm;
   if (grid > a.ntiles) grid = a.ntiles;
   launch_dep(conv_halo_kernel, (unsigned)grid, kHaloThreads, smem, st, tm, (const __nv_bfloat16 *)wpacked, a);
   cudaError_t e = cudaGetLastError();
@@ -1565,27 +1545,13 @@ struct PoolOut {
   int cstride, coff;
 };
 
-// The z-walk convolution (sepx_unet_zwfwd.inc): every layer the halo-staged
-// kernel takes whose three column blocks fit one MMA (3 x np <= 256) and whose
-// weights leave room for a ring of four slots (it measured 3.3 to 5.3 times as
-// fast on those).  Returns 1 where it does not apply: np 96 to 128 with cin up
-// to 24, np 96 or 112 with cin 32, and np 80 with cin 40 (226 KB of weights and
-// halo fit, 249 KB of weights and ring do not) stay on the halo-staged kernel.
+// The z-walk convolution, in the layers of zwalk_plan (else 1).
 int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
                const void *wpacked, const float *bias, int cout, int np, int relu, void *y, int y_cstride,
                int y_coff, float *yf, const float *resid, View mask, int *err, const PoolOut *pool, cudaStream_t st) {
-  if (3 * np > 256) return 1;
-  if (pool && (D % 2 || H % 2 || W % 2)) return 1;
   if (unet_dev_init()) return -1;
-  auto fit = [&](int nslot) {
-    const size_t sm = zf_smem_bytes(cin, np, nslot);
-    if (sm > kHaloMaxSmem) return 0;
-    return (int)(g_smem_per_sm / (((sm + 127) / 128) * 128 + g_smem_reserved));
-  };
-  // two CTAs per SM (each with half the tensor memory) where two rings fit,
-  // so that one's start-up and last planes overlap the other's MMAs
-  const int per_sm = std::min(fit(kZfMinSlots), 2);
-  if (per_sm < 1) return 1;
+  ZwalkPlan pl;
+  if (!zwalk_plan(g_dev, nb, D, H, W, cin, np, pool != nullptr, pl)) return 1;
   CUtensorMap tm;
   const bool thin = cin == 8 && x_cstride == 8 && !pool;
   if (thin) {
@@ -1621,48 +1587,8 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
   a.pool = pool ? pool->p : nullptr;
   a.pool_cstride = pool ? pool->cstride : 0;
   a.pool_coff = pool ? pool->coff : 0;
-  a.nslot = kZfMinSlots;
-  while (a.nslot < kZfMaxSlots && fit(a.nslot + 1) >= per_sm) a.nslot++;
-  a.ty = (H + kTileY - 1) / kTileY;
-  a.tx = (W + kTileX - 1) / kTileX;
-  const long long cols = (long long)nb * a.ty * a.tx;
-  if (cols * D >= (1LL << 31)) return 1;
-  // planes per window: the accumulators fill this CTA's share of the 512
-  // tensor-memory columns at most; among those the count with the least MMA
-  // time on the busiest CTA (an MMA of N columns takes max(32 + N / 4, N / 2)
-  // cycles; the two planes outside the window feed one column block, the two
-  // inside its ends two)
-  const long long slots = (long long)g_num_sms * per_sm;
-  const int zmax = std::min(std::min(kZfMaxZ, D), (512 / per_sm) / np);
-  auto mma_cycles = [&](int zc) {   // a tap's MMAs over a window
-    double c = 0;
-    for (int p = 0; p < zc + 2; p++) {
-      const int blk = std::min(p, zc - 1) - std::max(p - 2, 0) + 1;
-      c += std::max(32.0 + 0.25 * np * blk, 0.5 * np * blk);
-    }
-    return c;
-  };
-  double best = 1e300;
-  a.zc = 1;
-  const int zstep = pool ? 2 : 1;   // (pooled: windows of whole plane pairs)
-  for (int zc = zstep; zc <= zmax; zc += zstep) {
-    const long long items = cols * ((D + zc - 1) / zc);
-    const long long per = (items + slots - 1) / slots;
-    const double cost = (double)per * mma_cycles(zc);
-    if (cost < best) {
-      best = cost;
-      a.zc = zc;
-    }
-  }
-  a.nzc = (D + a.zc - 1) / a.zc;
-  a.zc = (D + a.nzc - 1) / a.nzc;   // the same windows, evenly filled
-  if (pool) {
-    a.zc += a.zc & 1;
-    a.nzc = (D + a.zc - 1) / a.zc;
-  }
-  a.nitems = (int)(cols * a.nzc);
-  a.late_from = g_num_sms;
-  a.late = (int)(0.75 * 9 * (halo_groups(cin) / 2) * mma_cycles(a.zc));
+  a.nslot = pl.nslot; a.ty = pl.ty; a.tx = pl.tx; a.zc = pl.zc; a.nzc = pl.nzc; a.nitems = pl.nitems;
+  a.late_from = pl.late_from; a.late = pl.late;
   const int form = pool ? 1 : (thin ? 2 : 0);
   const auto kern = pool ? conv_zwalk_kernel<true, false>
                          : (thin ? conv_zwalk_kernel<false, true> : conv_zwalk_kernel<false, false>);
@@ -1675,78 +1601,22 @@ int conv_zwalk(const void *x, int x_cstride, int x_coff, int nb, int D, int H, i
     if (e != cudaSuccess) return set_error("unet conv: %s", cudaGetErrorString(e));
     attr[form] = true;
   }
-  const long long grid = std::min<long long>(a.nitems, slots);
-  launch_dep(kern, (unsigned)grid, kZfThreads, zf_smem_bytes(cin, np, a.nslot), st, tm, tw, a);
+  launch_dep(kern, (unsigned)pl.grid, kZfThreads, pl.smem, st, tm, tw, a);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
 }
 
-// The convolution with streamed weights (sepx_unet_kstream.inc): 3x3x3 layers
-// whose weights do not fit in shared memory or whose planes are smaller than a
-// tile, where channels come in pairs of groups (a K16 step stays in one tap),
-// the planes a K range reads fit in shared memory, staging them moves at most
-// 0.4 of what the gather kernel copies for the range and the tile's real
-// voxels, and a range's MMAs take at least 1400 cycles (an item's fixed costs).
-// Measured (gather -> this, us a call; share staged, cycles): 112 -> 48 on 32^3
-// voxels 91 -> 30 (0.20, 4224), 64 -> 64 on 40 x 12 x 40 26.4 -> 17.5 (0.26,
-// 2592), 32 -> 48 on 116 x 12 x 122 83 -> 61 (0.22, 2376), 48 -> 16 on 68 x 12 x
-// 40 27.9 -> 22.5 (0.26, 1584); at the lines 112 -> 48 on 2 x 30 x 9 x 51 53.5 ->
-// 53.3 (0.36), 48 -> 64 on 30 x 9 x 40 18.4 -> 18.4 (1152); short of them 16 ->
-// 16 on 2 x 14 x 9 x 100 11.6 -> 20.9 (0.33, 576), 16 -> 32 on 50 x 9 x 100 15.9
-// -> 26.6 (1080), 64 -> 64 on 16^3, the kernels, 10.5 -> 11.2 (0.47).
-// Returns 1 where it does not apply.
+// The convolution with streamed weights, in the layers of kstream_span and kstream_plan (else 1).
 int conv_kstream(View x, int nb, int D, int H, int W, int cin, const void *wpacked, const float *bias, int cout,
                  int np, int relu, void *y, int y_cstride, int y_coff, float *yf, const float *resid, View mask,
                  int *err, int splits, int kper, float *kpart, cudaStream_t st) {
-  if (cin % 16 || cin / 8 > kKsMaxGroups) return 1;
-  KsArgs a;
-  a.ty = (H + kTileY - 1) / kTileY;
-  a.tx = (W + kTileX - 1) / kTileX;
-  const long long cols = (long long)nb * a.ty * a.tx;
-  if (cols * D * splits >= (1LL << 31)) return 1;
-  // planes of one output plane that any range reads
-  int span = 1;
-  const int per9 = 9 * (cin / 16);
-  for (int s = 0; s < splits; s++) {
-    const int k0 = s * kper * (kKC / 16), k1 = std::min(k0 + kper * (kKC / 16), 3 * per9);
-    span = std::max(span, (k1 - 1) / per9 - k0 / per9 + 1);
-  }
-  const double staged = (double)cols * D * span * (kHaloX * kHaloY) * cin, gathered = (double)nb * D * H * W * kper * kKC;
-  const int steps = std::min(kper * (kKC / 16), 3 * per9);
-  if (2.5 * staged > gathered || steps * std::max(32.0 + 0.25 * np, 0.5 * np) < 1400) return 1;
+  const int span = kstream_span(nb, D, H, W, cin, np, splits, kper);
+  if (!span) return 1;
   if (unet_dev_init()) return -1;
-  auto fit = [&](int nring, int nw) {
-    const size_t sm = ks_smem_bytes(cin, np, nring, nw);
-    if (sm > kHaloMaxSmem) return 0;
-    return std::min((int)(g_smem_per_sm / ((sm + 127) / 128 * 128 + g_smem_reserved)), 2);
-  };
-  // two CTAs per SM where the planes and two weight slots leave room for them
-  const int want = std::max(fit(span, 2), 1);
-  a.nw = kKsMaxW;
-  while (a.nw > 2 && fit(span, a.nw) < want) a.nw--;
-  const int per_sm = fit(span, a.nw);
-  if (!per_sm) return 1;
-  a.nring = span;
-  while (a.nring < kKsMaxRing && fit(a.nring + 1, a.nw) >= per_sm) a.nring++;
-  // output planes of an item: all ranges of a split layer are items already;
-  // else the count with the fewest planes on the busiest CTA (an item's first
-  // planes cost about half an output plane's MMAs)
-  const long long slots = (long long)g_num_sms * per_sm;
-  a.zc = 1;
-  if (splits == 1) {
-    double best = 1e300;
-    for (int zc = 1; zc <= D; zc++) {
-      const long long items = cols * ((D + zc - 1) / zc);
-      const double c = (double)((items + slots - 1) / slots) * (zc + 0.5);
-      if (c < best) {
-        best = c;
-        a.zc = zc;
-      }
-    }
-  }
-  a.nzc = (D + a.zc - 1) / a.zc;
-  a.zc = (D + a.nzc - 1) / a.nzc;   // the same runs, evenly filled
-  a.nitems = (int)(cols * a.nzc * splits);
+  KstreamPlan pl;
+  if (!kstream_plan(g_dev, nb, D, H, W, cin, np, splits, span, pl)) return 1;
+  KsArgs a;
+  a.nring = pl.nring; a.nw = pl.nw; a.ty = pl.ty; a.tx = pl.tx; a.zc = pl.zc; a.nzc = pl.nzc; a.nitems = pl.nitems;
   a.x = x; a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.np = np; a.relu = relu;
   a.wp = (const __nv_bfloat16 *)wpacked; a.bias = bias;
   a.y = (__nv_bfloat16 *)y; a.y_cstride = y_cstride; a.y_coff = y_coff;
@@ -1762,8 +1632,7 @@ int conv_kstream(View x, int nb, int D, int H, int W, int cin, const void *wpack
     if (e != cudaSuccess) return set_error("unet conv: %s", cudaGetErrorString(e));
     attr = true;
   }
-  launch_dep(conv_kstream_kernel, (unsigned)std::min<long long>(a.nitems, slots), kKsThreads, ks_smem_bytes(cin, np,
-             a.nring, a.nw), st, a);
+  launch_dep(conv_kstream_kernel, (unsigned)pl.grid, kKsThreads, pl.smem, st, a);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : set_error("unet conv: %s", cudaGetErrorString(e));
 }
@@ -1773,91 +1642,26 @@ int conv_kstream(View x, int nb, int D, int H, int W, int cin, const void *wpack
 int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
                     const void *dy, int dy_cstride, int dy_coff, int cout, float *dw, float *db, int *err,
                     cudaStream_t st) {
-  const int ngi = cin / 8, ngo = (cout + 7) / 8;
-  if (!g_halo_enabled || g_wgrad_form < 2 || ngi > 14 || ngo > 8) return 1;
+  if (!g_halo_enabled || g_wgrad_form < 2 || !ring_applies(cin, cout)) return 1;
   if (unet_dev_init()) return -1;
+  RingPlan pl;
+  if (!ring_plan(g_dev, nb, D, H, W, cin, cout, pl)) return 1;
   RgArgs a;
   a.x = View{(const __nv_bfloat16 *)x, x_cstride, x_coff};
   a.dy = View{(const __nv_bfloat16 *)dy, dy_cstride, dy_coff};
   if (reinterpret_cast<uintptr_t>(a.x.p + x_coff) % 16 || reinterpret_cast<uintptr_t>(a.dy.p + dy_coff) % 16)
     return set_error("unet wgrad: view not 16-byte aligned");
-  a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.ngo = ngo;
-  a.ncb = (ngi + 1) / 2;
-  a.pw = cout <= 16 ? 16 : (cout <= 32 ? 32 : 64);
-  a.nmbt = a.pw == 64 ? 2 : 1;
-  a.stacked = 48 * a.ncb <= 256;
-  a.n = a.stacked ? 48 * a.ncb : 16 * a.ncb;
-  const int ncn = a.stacked ? a.n : 3 * a.n;
-  // as much of a tile's work per CTA as the tensor memory holds: fewer CTAs
-  // read the same planes
-  a.nsy = a.nmbt * 3 * ncn <= 512 ? 3 : 1;
-  a.nmb = a.nmbt * a.nsy * ncn <= 512 ? a.nmbt : 1;
-  if (a.nmb * a.nsy * ncn > 512) return 1;
-  // One CTA per SM with the longest ring that fits (four planes at least).  Two
-  // with shorter rings take 41 instead of 47 us for 16 -> 16 channels on 4 x
-  // 64^3 voxels alone, but 1155 instead of 1137 in the training step, where a
-  // data gradient's CTAs then find no room beside them and twice as many
-  // partials are added.
-  auto fits = [&](int na, int nring) { return rg_smem_bytes(a.ncb, a.pw, na, nring) <= kHaloMaxSmem; };
-  a.na = fits(kRgMaxA, 8) ? kRgMaxA : (fits(3, 6) ? 3 : 2);
-  a.nring = kRgMaxRing;
-  while (a.nring > 4 && !fits(a.na, a.nring)) a.nring--;
-  if (!fits(a.na, a.nring)) return 1;
+  a.nb = nb; a.D = D; a.H = H; a.W = W; a.cin = cin; a.cout = cout; a.ngo = pl.ngo;
+  a.ncb = pl.ncb; a.pw = pl.pw; a.nmbt = pl.nmbt; a.stacked = pl.stacked; a.n = pl.n; a.nsy = pl.nsy; a.nmb = pl.nmb;
+  a.na = pl.na; a.nring = pl.nring;
   CUtensorMap tmx, tmy;
   if (encode_view(&tmx, a.x.p, a.x.cstride, a.x.coff, cin, nb, D, H, W, 8, kHaloY, 1, "wgrad", 16,
                   CU_TENSOR_MAP_SWIZZLE_32B) ||
-      encode_view(&tmy, a.dy.p, a.dy.cstride, a.dy.coff, 8 * ngo, nb, D, H, W, 10, 16, 1, "wgrad", a.pw,
+      encode_view(&tmy, a.dy.p, a.dy.cstride, a.dy.coff, 8 * a.ngo, nb, D, H, W, 10, 16, 1, "wgrad", a.pw,
                   a.pw == 16 ? CU_TENSOR_MAP_SWIZZLE_32B
                              : (a.pw == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B)))
     return -1;
-  a.ty = (H + 15) / 16;
-  a.tx = (W + 2 + 7) / 8;
-  const int njob = (3 / a.nsy) * (a.nmbt / a.nmb);
-  const int slots = std::max(1, g_num_sms / njob);
-  // planes per window: the run with the least work on the busiest CTA (a
-  // window loads two planes more than it has tiles; counted half a tile each)
-  const long long cols = (long long)nb * a.ty * a.tx;
-  if (cols * D >= (1LL << 31)) return 1;
-  double best = 1e300;
-  for (int zc = 1; zc <= D; zc++) {
-    const int nzc = (D + zc - 1) / zc;
-    if (zc > 1 && (D + nzc - 1) / nzc != zc) continue;   // windows as even as the count allows
-    const long long per = (cols * nzc + slots - 1) / slots;
-    const double cost = (double)per * (zc + 1.0);
-    if (cost <= best) {
-      best = cost;
-      a.zc = zc;
-      a.nzc = nzc;
-    }
-  }
-  a.nitems = (int)(cols * a.nzc);
-  a.groups = std::min(a.nitems, slots);
-  // The tensor cores truncate as they add: a chain of n MMAs (8 a tile) into
-  // one accumulator loses about 1.5e-8 n of a sum, in one direction.  So the
-  // accumulators are read out, and added in FP32 to the CTA's partial sums,
-  // once they have taken the tiles of a chain that `acc` accumulators per SM
-  // would leave each, `least` at least.  The numbers are those of the forms
-  // that ran these layers before (one to four CTAs an SM; the gather kernel's
-  // splits), whose errors are the bound.  Relative L2 error of one read-out ->
-  // of these (and time, us): 8 -> 16 channels on 4 x 64^3 voxels 7.2e-6 ->
-  // 1.4e-6 (47 -> 55), 32 -> 48 2.2e-5 -> 3.8e-6 (152 -> 170), 112 -> 48 on 2 x
-  // 64^3 2.1e-5 -> 7.1e-6 (207 -> 216), 32 -> 32 on 4 x 32^3 8.2e-7 -> 4.0e-7
-  // (23 -> 29); a training step on 4 x 64^3 1018 -> 1091.
-  double acc;
-  int least;
-  if (njob == 1) {
-    acc = a.pw == 16 && a.ncb == 1 ? (cin == 8 ? 4.0 : 2.0) : 1.0;
-    least = a.pw == 16 && a.ncb == 1 ? 2 : 4;
-  } else if (cout <= 40) {
-    acc = a.pw == 64 ? 1.43 : 0.72;
-    least = 2;
-  } else {
-    acc = 10.0 / ((27 * cin + 127) / 128);
-    least = 8;
-  }
-  const int run = (a.nitems + a.groups - 1) / a.groups * a.zc;   // tiles of the busiest CTA
-  const int nout = (int)std::ceil(run / std::max((double)least, 1.1 * (double)(cols * D) / (g_num_sms * acc)));
-  a.seg = (run + nout - 1) / nout;
+  a.ty = pl.ty; a.tx = pl.tx; a.zc = pl.zc; a.nzc = pl.nzc; a.nitems = pl.nitems; a.groups = pl.groups; a.seg = pl.seg;
   a.err = err;
   // 16, 32, 64 rows' channels x (three sy stacked, one sy stacked, one sy per dz)
   const decltype(&conv_wgrad_ring_kernel<16, 3, true>) kerns[9] = {
@@ -1880,7 +1684,7 @@ int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int
   if (unet_scratch(kScrGrad, (size_t)a.groups * (size_t)(n + cout), &scr, st)) return -1;
   a.part = scr;
   a.bpart = db ? scr + (size_t)a.groups * n : nullptr;
-  kern<<<(unsigned)(a.groups * njob), kRgThreads, rg_smem_bytes(a.ncb, a.pw, a.na, a.nring), st>>>(tmx, tmy, a);
+  kern<<<(unsigned)(a.groups * pl.njob), kRgThreads, pl.smem, st>>>(tmx, tmy, a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error("unet wgrad: %s", cudaGetErrorString(e));
   wg_reduce(a.part, a.groups, n, dw, a.bpart, cout, db, st);
@@ -1935,7 +1739,7 @@ int conv_wgrad_tma(const void *x, int x_cstride, int x_coff, int nb, int D, int 
     return -1;
   uint32_t ncols = 32;
   while (ncols < (uint32_t)(ndz * np)) ncols <<= 1;
-  int per_sm = (int)(g_smem_per_sm / (((smem + 127) / 128) * 128 + g_smem_reserved));
+  int per_sm = (int)(g_dev.smem_per_sm / (((smem + 127) / 128) * 128 + g_dev.smem_reserved));
   if (per_sm < 1) return 1;
   if (per_sm * (int)ncols > 512) per_sm = 512 / (int)ncols;
   const int nzg = 3 / ndz;
@@ -1946,7 +1750,7 @@ int conv_wgrad_tma(const void *x, int x_cstride, int x_coff, int nb, int D, int 
   a.tx = (W + 2 + 7) / 8;
   a.ntiles = (long long)nb * D * a.ty * a.tx;
   if (a.ntiles >= (1LL << 31)) return 1;
-  a.groups = (g_num_sms * per_sm) / nzg;
+  a.groups = (g_dev.num_sms * per_sm) / nzg;
   if (a.groups > a.ntiles) a.groups = (int)a.ntiles;
   if (a.groups < 1) a.groups = 1;
   a.stages = stages;
@@ -2076,26 +1880,20 @@ int conv_any(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int
   const long long V = (long long)nb * D * H * W;
   if (V >= (1LL << 31) || (long long)H * W * x_cstride >= (1LL << 30))
     return set_error("unet conv: volume too large (%lld voxels)", V);
-  if (ntap == 27 && H >= kTileY && W >= kTileX && halo_groups(cin) / 2 <= kMaxPairs && g_halo_enabled) {
-    // packed weights of the 27 taps, plus one K group for an odd group count
-    // (the packing pads with zeros up to a multiple of 8 groups, and 27 * an
-    // odd count is never one)
-    const int ngc = cin / 8;
-    const uint32_t wbytes = (uint32_t)((27 * ngc + (ngc & 1)) * (np / 8) * 128);
-    if (halo_smem_bytes(cin, wbytes, 1) <= kHaloMaxSmem) {
-      int rc = 1;
-      if (pool) {
-        rc = conv_zwalk(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y, y_cstride, y_coff, yf,
-                        resid, mv, err, pool, (cudaStream_t)stream);
-        if (!rc) *pooled = 1;
-      }
-      if (rc > 0)
-        rc = conv_zwalk(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y, y_cstride, y_coff, yf,
-                        resid, mv, err, nullptr, (cudaStream_t)stream);
-      if (rc <= 0) return rc;
-      return conv_halo(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, wbytes, bias, cout, np, relu, y,
-                       y_cstride, y_coff, yf, resid, mv, err, (cudaStream_t)stream);
+  uint32_t wbytes;
+  if (ntap == 27 && g_halo_enabled && halo_applies(H, W, cin, np, &wbytes)) {
+    int rc = 1;
+    if (pool) {
+      rc = conv_zwalk(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y, y_cstride, y_coff, yf,
+                      resid, mv, err, pool, (cudaStream_t)stream);
+      if (!rc) *pooled = 1;
     }
+    if (rc > 0)
+      rc = conv_zwalk(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, bias, cout, np, relu, y, y_cstride, y_coff, yf,
+                      resid, mv, err, nullptr, (cudaStream_t)stream);
+    if (rc <= 0) return rc;
+    return conv_halo(x, x_cstride, x_coff, nb, D, H, W, cin, wpacked, wbytes, bias, cout, np, relu, y,
+                     y_cstride, y_coff, yf, resid, mv, err, (cudaStream_t)stream);
   }
   if (ntap == 1 && g_halo_enabled && ((cin == 16 && cout == 1 && !y) || (cin == 8 && cout == 16))) {
     View xv{(const __nv_bfloat16 *)x, x_cstride, x_coff};
