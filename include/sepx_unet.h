@@ -57,10 +57,10 @@ int sepx_unet_conv_fwd_masked(const void *x, int x_cstride, int x_coff, int nb, 
  * kernels.  Returns the previous setting. */
 int sepx_unet_set_halo(int enable);
 /* Weight-gradient kernel choice (with the halo-staged kernels enabled):
- * 2 (default) the ring tap-stacked kernel (cin <= 112, cout <= 64), else
- * the per-tile tap-stacked kernel (cin <= 80, cout <= 40), else the gather
- * kernel; 1 the per-tile kernel, else gather; 0 gather.  Returns the
- * previous choice, or -1 for another value. */
+ * 2 (default) the ring tap-stacked kernel (cin <= 112, cout <= 64), else the
+ * gather kernel; 1 the per-tile tap-stacked kernel (cin <= 80, cout <= 40), the
+ * same sums by another schedule, to compare with, else gather; 0 gather.
+ * Returns the previous choice, or -1 for another value. */
 int sepx_unet_set_wgrad_form(int form);
 /* The BF16 convolution and the 2x2x2 average of its output into the view p
  * (D, H, W even): the same bits as sepx_unet_conv_fwd, then sepx_unet_avgpool,

@@ -1401,7 +1401,7 @@ int check_conv_args(int cin, int cstride, int coff, int cout, int ntap) {
 int np_of(int cout) { return ((cout + 15) / 16) * 16; }
 
 bool g_halo_enabled = true;
-int g_wgrad_form = 2;   // 2: ring, else per-tile TMA, else gather; 1: per-tile TMA, else gather; 0: gather
+int g_wgrad_form = 2;   // 2: ring, else gather; 1: per-tile TMA, else gather; 0: gather
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 UnetDev g_dev;
 
@@ -1642,7 +1642,7 @@ int conv_kstream(View x, int nb, int D, int H, int W, int cin, const void *wpack
 int conv_wgrad_ring(const void *x, int x_cstride, int x_coff, int nb, int D, int H, int W, int cin,
                     const void *dy, int dy_cstride, int dy_coff, int cout, float *dw, float *db, int *err,
                     cudaStream_t st) {
-  if (!g_halo_enabled || g_wgrad_form < 2 || !ring_applies(cin, cout)) return 1;
+  if (!g_halo_enabled || g_wgrad_form != 2 || !ring_applies(cin, cout)) return 1;
   if (unet_dev_init()) return -1;
   RingPlan pl;
   if (!ring_plan(g_dev, nb, D, H, W, cin, cout, pl)) return 1;
@@ -1699,7 +1699,7 @@ int conv_wgrad_tma(const void *x, int x_cstride, int x_coff, int nb, int D, int 
                    const void *dy, int dy_cstride, int dy_coff, int cout, float *dw, float *db, int *err,
                    cudaStream_t st) {
   const int ngi = cin / 8, ngo = (cout + 7) / 8;
-  if (!g_halo_enabled || g_wgrad_form < 1 || 3 * ngo > 16 || 3 * ngi + 1 > 32) return 1;
+  if (!g_halo_enabled || g_wgrad_form != 1 || 3 * ngo > 16 || 3 * ngi + 1 > 32) return 1;
   if (unet_dev_init()) return -1;
   const int np = ((8 * (3 * ngi + 1)) + 15) / 16 * 16;
   const uint32_t a_bytes = 3u * ngo * kWgBox;
