@@ -549,14 +549,12 @@ int loop_rtm_adjoint(int jt, int npts, int nt) {
   P.nrec = G.rec_nx * G.rec_ny;
   Rows2Maps H;
   H.vel_h = G.vel.tm_h2;
-  // A launch per step for the source values costs about 5 us with its gap; the
-  // fused form costs the step kernel 2 % (a register for the next plane's
-  // slot): 128^3 model 10.24 -> 9.79 ms for 150 steps, 512 x 512 x 400 49.42
-  // -> 50.10 for 40.  The line is where both are about 4 us.
-  const PropGeom &gg = G.geom;
-  const long long cells = (long long)(gg.xe - gg.xb) * (gg.ye - gg.yb) * std::max(0, gg.ze - gg.zb);
-  const bool fused = npts > 0 && cells <= 32000000LL &&
-                     !(((G.rows2_mask >> kRtmAdj) & 1) && prop_step2_supported(kRtmAdj));
+  // The source values inside the next step cost it a register, a launch of their
+  // own after every step 4 us with its gap.  Launch -> fused, us a step: 64^3
+  // model 15.7 -> 13.8, 128^3 43.4 -> 43.4, 160^3 70.2 -> 66.3, 256 x 256 x 300
+  // 198.2 -> 193.9, 320^3 294.6 -> 289.6, 420 x 420 x 350 545.9 -> 542.1, 512 x
+  // 512 x 400 824.0 -> 818.2.  The two-row tile has no such form.
+  const bool fused = npts > 0 && !(((G.rows2_mask >> kRtmAdj) & 1) && prop_step2_supported(kRtmAdj));
   for (int it = nt - 1; it >= 0; it--) {
     const int id = it / jt, ii = it - id * jt;
     P.trc_id = id;

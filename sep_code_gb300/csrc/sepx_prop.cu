@@ -985,8 +985,11 @@ static cudaError_t launch_mode(const PropParams &P, dim3 grid, cudaStream_t st) 
   // descriptors, sponge table) while this step drains (128^3 model, source
   // propagation and adjoint: 10.59 -> 9.79 ms for 150 steps; 512 x 512 x 400:
   // 50.34 -> 50.10 for 40).  Not for the modes with z-queues in tensor memory:
-  // CTAs that start early crowd onto the SMs with room, and small grids ran
-  // slower (64^3 patch: 14.99 -> 15.61 ms), large ones no faster.
+  // CTAs that start early crowd onto the SMs with room, and which grids gain is
+  // uneven (us a step without -> with: Born forward on the 64^3 model 17.1 ->
+  // 17.3, 128^3 44.8 -> 43.6, 160^3 69.7 -> 72.6, 190^3 98.2 -> 101.5, 320^3 321.4 ->
+  // 319.0, 512 x 512 x 400 885.7 -> 884.2; linearised forward 19.3 -> 15.8, 48.5 ->
+  // 48.5, 74.9 -> 79.8, 108.6 -> 104.5, 339.1 -> 335.5, 906.0 -> 900.5).
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(kThreads);
