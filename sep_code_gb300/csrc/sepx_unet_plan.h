@@ -254,7 +254,8 @@ struct RingPlan {
   bool stacked;         // one MMA over (dz, c), or one per dz
   int n, ncols;         // its N; tensor-memory columns of a CTA
   int na, nring;        // dy and plane slots
-  int njob, ty, tx, zc, nzc, nitems, groups, seg;
+  int njob, ty, tx, zc, nzc, nitems, groups;
+  int seg;              // tiles an accumulator takes between two read-outs
   size_t smem;
 };
 
@@ -289,35 +290,20 @@ inline bool ring_plan(const UnetDev &dev, int nb, int D, int H, int W, int cin, 
   a.tx = (W + 2 + 7) / 8;
   const int njob = a.njob = (3 / a.nsy) * (a.nmbt / a.nmb);
   const int slots = std::max(1, dev.num_sms / njob);
-  // planes per window: the run with the least work on the busiest CTA (a
-  // window loads two planes more than it has tiles; counted half a tile each)
   const long long cols = (long long)nb * a.ty * a.tx;
   if (cols * D >= (1LL << 31)) return false;
-  double best = 1e300;
-  for (int zc = 1; zc <= D; zc++) {
-    const int nzc = (D + zc - 1) / zc;
-    if (zc > 1 && (D + nzc - 1) / nzc != zc) continue;   // windows as even as the count allows
-    const long long per = (cols * nzc + slots - 1) / slots;
-    const double cost = (double)per * (zc + 1.0);
-    if (cost <= best) {
-      best = cost;
-      a.zc = zc;
-      a.nzc = nzc;
-    }
-  }
-  a.nitems = (int)(cols * a.nzc);
-  a.groups = std::min(a.nitems, slots);
   // The tensor cores truncate as they add: a chain of n MMAs (8 a tile) into
   // one accumulator loses about 1.5e-8 n of a sum, in one direction.  So the
   // accumulators are read out, and added in FP32 to the CTA's partial sums,
   // once they have taken the tiles of a chain that `acc` accumulators per SM
-  // would leave each, `least` at least.  The numbers are those of the forms
-  // that ran these layers before (one to four CTAs an SM; the gather kernel's
-  // splits), whose errors are the bound.  Relative L2 error of one read-out ->
-  // of these (and time, us): 8 -> 16 channels on 4 x 64^3 voxels 7.2e-6 ->
-  // 1.4e-6 (47 -> 55), 32 -> 48 2.2e-5 -> 3.8e-6 (152 -> 170), 112 -> 48 on 2 x
-  // 64^3 2.1e-5 -> 7.1e-6 (207 -> 216), 32 -> 32 on 4 x 32^3 8.2e-7 -> 4.0e-7
-  // (23 -> 29); a training step on 4 x 64^3 1018 -> 1091.
+  // would leave each, `least` at least (the loads go on meanwhile).  The
+  // numbers are those of the forms that ran these layers before (one to four
+  // CTAs an SM; the gather kernel's splits), whose errors are the bound.
+  // Relative L2 error of one read-out -> of these (and time, us): 8 -> 16
+  // channels on 4 x 64^3 voxels 7.2e-6 -> 1.4e-6 (47 -> 53), 32 -> 48 2.2e-5 ->
+  // 3.8e-6 (152 -> 167), 112 -> 48 on 2 x 64^3 2.1e-5 -> 7.1e-6 (207 -> 216), 80 ->
+  // 32 on 4 x 32^3 2.4e-6 -> 7.1e-7 (33 -> 40), 32 -> 32 there 8.2e-7 -> 5.6e-7
+  // (23 -> 25); a training step on 4 x 64^3 1017 -> 1036.
   double acc;
   int least;
   if (njob == 1) {
@@ -330,9 +316,26 @@ inline bool ring_plan(const UnetDev &dev, int nb, int D, int H, int W, int cin, 
     acc = 10.0 / ((27 * cin + 127) / 128);
     least = 8;
   }
-  const int run = (a.nitems + a.groups - 1) / a.groups * a.zc;   // tiles of the busiest CTA
-  const int nout = (int)std::ceil(run / std::max((double)least, 1.1 * (double)(cols * D) / (dev.num_sms * acc)));
-  a.seg = (run + nout - 1) / nout;
+  const int most = (int)std::max((double)least, 1.1 * (double)(cols * D) / (dev.num_sms * acc));   // tiles of a chain
+  // planes per window: the run with the least work on the busiest CTA, in tiles
+  // (a window loads two planes more than it has tiles: half a tile each; a
+  // read-out takes as long as about five)
+  double best = 1e300;
+  for (int zc = 1; zc <= D; zc++) {
+    const int nzc = (D + zc - 1) / zc;
+    if (zc > 1 && (D + nzc - 1) / nzc != zc) continue;   // windows as even as the count allows
+    const long long per = (cols * nzc + slots - 1) / slots;
+    const int run = (int)(per * zc), nout = (run + most - 1) / most;
+    const double cost = (double)per * (zc + 1.0) + 5.0 * (nout - 1);
+    if (cost <= best) {
+      best = cost;
+      a.zc = zc;
+      a.nzc = nzc;
+      a.seg = (run + nout - 1) / nout;
+    }
+  }
+  a.nitems = (int)(cols * a.nzc);
+  a.groups = std::min(a.nitems, slots);
   a.ncols = a.nmb * a.nsy * ncn;
   a.smem = rg_smem_bytes(a.ncb, a.pw, a.na, a.nring);
   return true;
